@@ -205,8 +205,10 @@ size_t res_smem_cap(pyomgpu_ctx* c) {
   size_t stat = 0;
   std::vector<const void*> ks{cg_res_multi_kernel_ptr(false), cg_res_multi_kernel_ptr(true), cg_res32_kernel_ptr(16),
                               cg_res32_kernel_ptr(32)};
-  for (int k = 0; k < kResNP; k++)
+  for (int k = 0; k < kResNP; k++) {
     for (bool single : {false, true}) ks.push_back(cg_res_kernel_ptr(kResP[k], single));
+    ks.push_back(cg_res_sp_kernel_ptr(kResP[k]));
+  }
   for (const void* k : ks) {
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return 0;
@@ -243,9 +245,9 @@ int res_plan(pyomgpu_ctx* c) {
                                (int)cap) != cudaSuccess)
         return fail(PYOMGPU_ECUDA, "cannot reserve shared memory for the resident kernel");
   for (int k = 0; k < kResNP; k++)
-    if (cudaFuncSetAttribute(cg_res_trace_kernel_ptr(kResP[k]), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)cap) != cudaSuccess)
-      return fail(PYOMGPU_ECUDA, "cannot reserve shared memory for the resident kernel");
+    for (const void* f : {cg_res_trace_kernel_ptr(kResP[k]), cg_res_sp_kernel_ptr(kResP[k])})
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess)
+        return fail(PYOMGPU_ECUDA, "cannot reserve shared memory for the resident kernel");
   for (bool single : {false, true}) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_res_kernel_ptr(R.p, single), kResThreads,
@@ -253,6 +255,11 @@ int res_plan(pyomgpu_ctx* c) {
         per_sm < 1)
       return PYOMGPU_OK;
   }
+  int per_sm_sp = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_sp, cg_res_sp_kernel_ptr(R.p), kResThreads, R.smem) !=
+          cudaSuccess ||
+      per_sm_sp < 1)
+    return PYOMGPU_OK;
   const int nb = R.npx * R.npy;
   if (int rc = dalloc(&R.hx, 8 * c->g.size())) return rc;  // two record buffers
   if (int rc = dalloc(&R.slots, (size_t)4 * (nb + 1) * kResSlotWords)) return rc;
@@ -265,9 +272,10 @@ bool use_resident(pyomgpu_ctx* c) {
   return res_plan(c) == PYOMGPU_OK && c->resd.ok;
 }
 
-// The streamfunction solve in the on-chip-resident kernel (cg_res.cu).
-int run_cg_res(pyomgpu_ctx* c, const double* forc_dev, double eps, int max_it, double rtol, pyomgpu_solve_info* info,
-               cudaStream_t st) {
+// The streamfunction solve (or, with surf_press, congrad_surf_press) in the
+// on-chip-resident kernel (cg_res.cu).
+int run_cg_res(pyomgpu_ctx* c, bool surf_press, const double* forc_dev, double eps, int max_it, double rtol,
+               pyomgpu_solve_info* info, cudaStream_t st) {
   auto& R = c->resd;
   const size_t bytes = c->g.size() * sizeof(double);
   const int nb = R.npx * R.npy;
@@ -279,7 +287,7 @@ int run_cg_res(pyomgpu_ctx* c, const double* forc_dev, double eps, int max_it, d
   CK(cudaMemsetAsync(R.hx, 0xFF, 8 * c->g.size() * sizeof(double), st));
   CGResParams P{};
   P.g = c->g;
-  P.op = c->sf.dev();
+  P.op = surf_press ? c->sp.dev() : c->sf.dev();
   P.forc = forc_dev;
   P.sol = c->sol;
   P.res = c->res;
@@ -301,16 +309,21 @@ int run_cg_res(pyomgpu_ctx* c, const double* forc_dev, double eps, int max_it, d
   P.tag_gen = R.tag_gen;  // tags of this solve's slots and records differ from the previous solve's
   R.tag_gen = (R.tag_gen + 1u) % 4095u;
   P.out = c->d_result;
-  const bool trace = R.trace_nit > 0 && c->cg_kernel != 3;
+  const bool trace = R.trace_nit > 0 && c->cg_kernel != 3 && !surf_press;
   P.trace = trace ? R.trace : nullptr;
   P.trace_it0 = R.trace_it0;
   P.trace_nit = trace ? R.trace_nit : 0;
   void* args[] = {&P};
+  const bool cyclic = c->g.cyclic_x || c->g.cyclic_y;
+  if (surf_press && cyclic) launch_halo_offset(c->g, c->sol, c->s0, st);
   CK(cudaEventRecord(c->e0, st));
   const bool single = c->cg_kernel == 3;  // automatic: the two-reduction form (the reference's recurrences)
-  const void* kern = trace ? cg_res_trace_kernel_ptr(R.p) : cg_res_kernel_ptr(R.p, single);
+  const void* kern = surf_press ? cg_res_sp_kernel_ptr(R.p)
+                     : trace    ? cg_res_trace_kernel_ptr(R.p)
+                                : cg_res_kernel_ptr(R.p, single);
   CK(cudaLaunchCooperativeKernel(kern, dim3(nb), dim3(kResThreads), args, R.smem, st));
   CK(cudaEventRecord(c->e1, st));
+  if (surf_press && cyclic) launch_halo_restore(c->g, c->sol, c->s0, st);
   return finish_cg(c, info, st);
 }
 
@@ -397,7 +410,9 @@ int run_cg_res32(pyomgpu_ctx* c, const OpDev<float>& op, const float* b, float* 
 // Fortran-layout device forcing.  Fills info (iterations, status, timing).
 int run_cg_ref(pyomgpu_ctx* c, bool surf_press, const double* forc_dev, double eps, int max_it, double rtol,
                pyomgpu_solve_info* info, cudaStream_t st) {
-  if (!surf_press && use_resident(c)) return run_cg_res(c, forc_dev, eps, max_it, rtol, info, st);
+  // congrad_surf_press runs on chip too wherever the grid fits and the mask is 0/1 (1440x720: 51.2 ms tiled)
+  if ((!surf_press || c->sp_mask01) && use_resident(c))
+    return run_cg_res(c, surf_press, forc_dev, eps, max_it, rtol, info, st);
   const OpBuf& op = surf_press ? c->sp : c->sf;
   const size_t bytes = c->g.size() * sizeof(double);
   CK(cudaMemsetAsync(c->ctl, 0, sizeof(SyncCtl), st));
@@ -1455,6 +1470,7 @@ int32_t pyomgpu_ctx_create(const pyomgpu_grid* gr, pyomgpu_ctx** out) {
   if (c->have_sp) {
     if ((rc = upload(&c->hu, gr->hu, n2)) || (rc = upload(&c->hv, gr->hv, n2)) || (rc = upload(&c->mT, gr->maskT_top, n2)))
       return bail(rc);
+    c->sp_mask01 = std::all_of(gr->maskT_top, gr->maskT_top + n2, [](double m) { return m == 0.0 || m == 1.0; });
   }
   const size_t P = c->g.size();
   for (OpBuf* op : {&c->sf, &c->sp}) {

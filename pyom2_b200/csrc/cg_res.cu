@@ -295,6 +295,7 @@ struct ResCtl {
 };
 constexpr int kRun = 0, kDoneOk = 1, kDoneErr = 2, kNeedMaxp = 3;
 constexpr int kStepInit = 0, kStepA = 1, kStepB = 2, kStepInitD = 3, kStepIter = 4, kStepMaxp = 5;
+constexpr int kStepInitP = 6, kStepAP = 7, kStepBP = 8;  // congrad_surf_press
 
 __device__ __forceinline__ void ctl_stop(ResCtl& C, int act, int status) {
   C.act = act;
@@ -369,6 +370,79 @@ __device__ void ctl_after_b(ResCtl& C, const CGResParams& P, const double* v) {
   C.beta = beta_next;
   C.n += 1;
   ctl_begin(C, P);
+}
+
+// congrad_surf_press (solve_pressure.f90:163-232), as cg_ref_kernel<true> runs
+// it: products weighted by maskT, no preconditioner, and a convergence test of
+// iteration n that needs max|p| of the direction formed after it, so it is
+// decided at the next sweep A.
+// v = (res, res), (forc, forc) over maskT
+__device__ void ctl_init_sp(ResCtl& C, const CGResParams& P, const double* v) {
+  C.beta = v[0];
+  C.bb = v[1];
+  C.rtol2bb = P.rtol * P.rtol * C.bb;
+  C.betam1 = 1.0;
+  C.betamin = C.step1 = C.est = C.bq = C.alpha = 0.0;
+  C.n = 0;
+  C.status = PYOMGPU_OK;
+  C.act = kRun;
+  C.stop_after = 0;
+  if (C.beta == 0.0) return ctl_stop(C, kDoneOk, PYOMGPU_OK);  // solve_pressure.f90:174-177
+  C.n = 1;
+  if (P.max_it < 1) return ctl_stop(C, kDoneErr, PYOMGPU_MAXITER);
+}
+
+// v = (p, Ap), max|p| of the direction of iteration C.n; C.alpha and C.beta are still iteration n-1's step and
+// its (res, res)
+__device__ void ctl_after_a_sp(ResCtl& C, const CGResParams& P, const double* v) {
+  const double sAs = v[0], smax = v[1];
+  if (C.n > 1) {  // convergence test of iteration n-1 (solve_pressure.f90:209-226)
+    const int m = C.n - 1;
+    const double step = fabs(C.alpha) * smax;
+    bool stop = false;
+    if (m == 1) {
+      C.step1 = step;
+      C.est = step;
+      stop = step < P.eps;
+    } else if (step < P.eps) {
+      const double rate = exp(log(step / C.step1) / (double)(m - 1));
+      C.est = step * rate / (1.0 - rate);
+      stop = C.est < P.eps;
+    }
+    if (stop) {
+      C.n = m;
+      return ctl_stop(C, kDoneOk, PYOMGPU_OK);
+    }
+    if (C.est != C.est) {
+      C.n = m;
+      return ctl_stop(C, kDoneErr, PYOMGPU_NAN);
+    }
+    if (P.rtol > 0.0 && (C.bb > 0.0 ? C.beta <= C.rtol2bb : C.beta == 0.0)) {
+      C.est = sqrt(C.beta);
+      C.n = m;
+      return ctl_stop(C, kDoneOk, PYOMGPU_OK);
+    }
+    if (m >= P.max_it) {  // solve_pressure.f90:228-229
+      C.n = P.max_it + 1;
+      return ctl_stop(C, kDoneErr, PYOMGPU_MAXITER);
+    }
+  }
+  if (sAs == 0.0) return ctl_stop(C, kDoneOk, PYOMGPU_OK);  // :185
+  C.alpha = C.beta / sAs;
+}
+
+// v = (res, res) over maskT of the updated residual
+__device__ void ctl_after_b_sp(ResCtl& C, const double* v) {
+  const double rsnew = v[0];
+  C.bq = rsnew / C.beta;  // p = res + rsnew/rsold*p (solve_pressure.f90:190)
+  C.beta = rsnew;
+  if (C.n == 1) {  // :197-205
+    C.betamin = fabs(rsnew);
+  } else if (C.n > 2) {
+    C.betamin = fmin(C.betamin, fabs(rsnew));
+    if (fabs(rsnew) > 100.0 * C.betamin) return ctl_stop(C, kDoneErr, PYOMGPU_DIVERGED);
+  }
+  C.n += 1;
 }
 
 // Single-reduction form: with u = Z res, w = A u and the previous direction
@@ -775,6 +849,12 @@ __device__ __forceinline__ bool controller_epoch(const CGResParams& P, unsigned 
       ctl1_direction(C, P, out);
     else if (kStep == kStepIter)
       ctl1_iter(C, P, out);
+    else if (kStep == kStepInitP)
+      ctl_init_sp(C, P, out);
+    else if (kStep == kStepAP)
+      ctl_after_a_sp(C, P, out);
+    else if (kStep == kStepBP)
+      ctl_after_b_sp(C, out);
     else {  // kStepMaxp: the breakdown estimate, solve_streamfct.f90:262-266
       C.est = 100.0 * out[0];
       ctl_stop(C, kDoneOk, PYOMGPU_OK);
@@ -808,7 +888,11 @@ __device__ __forceinline__ void workers_sync() {
 // option for the psin solves).
 // FRESH: the reduction polls mix in atomic reads after a long wait
 // (controller_epoch), for the gangs of the multi-solve kernel.
-template <typename T, int P, bool TRACE, bool WGT = false, bool FRESH = false>
+// SP: congrad_surf_press.  The mask weight of a point (0 or 1; the caller
+// checks that) is one bit of a register, so TMEM holds no Z, the direction
+// starts from the residual itself and the diagonal term dcoef maskT is added
+// to the stencil.
+template <typename T, int P, bool TRACE, bool WGT = false, bool FRESH = false, bool SP = false>
 __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, double* sm, const uint32_t* s_tmem_p,
                                           ResCtl& C, double (*wred)[kResSlotWords]) {
   // points per TMEM chunk (FP64: tcgen05 .x16 / .x8, .x16 at P = 16 spills; FP32: .x8)
@@ -859,15 +943,16 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
     unsigned ep = 0;
     bool stopped_after_update = false;  // the stop decided before sweep B (C stays as the workers read it)
     __syncthreads();  // S1
-    bool ok = controller_epoch<4, 3, kStepInit, true, FRESH>(Pm, ep, bid, nb + (Pm.stall_extra ? 1 : 0), C, wred);
+    bool ok = controller_epoch<4, 3, SP ? kStepInitP : kStepInit, true, FRESH>(
+        Pm, ep, bid, nb + (Pm.stall_extra ? 1 : 0), C, wred);
     if (!__syncthreads_and(ok)) goto out;  // S2
     if (C.act == kRun) {
       for (unsigned trip = 0;; trip++) {
         unsigned long long* tr = threadIdx.x == 0 ? trace_row(trip) : nullptr;
         __syncthreads();  // S1: partials of sweep A
         if (TRACE && tr) tr[10] = globaltimer_ns();
-        ok = controller_epoch<2, 1, kStepA, true, FRESH>(Pm, ++ep, bid, nb, C, wred, nullptr,
-                                                        TRACE && tr ? tr + 11 : nullptr);
+        ok = controller_epoch<2, 1, SP ? kStepAP : kStepA, true, FRESH>(Pm, ++ep, bid, nb, C, wred, nullptr,
+                                                                       TRACE && tr ? tr + 11 : nullptr);
         if (!__syncthreads_and(ok)) goto out;  // S2
         if (C.act != kRun) break;
         if (C.stop_after) {  // the workers finish sweep B and stop
@@ -876,8 +961,8 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
         }
         __syncthreads();  // S1: partials of sweep B
         if (TRACE && tr) tr[14] = globaltimer_ns();
-        ok = controller_epoch<2, -1, kStepB, true, FRESH>(Pm, ++ep, bid, nb, C, wred, nullptr,
-                                                   TRACE && tr ? tr + 15 : nullptr);
+        ok = controller_epoch<SP ? 1 : 2, -1, SP ? kStepBP : kStepB, true, FRESH>(
+            Pm, ++ep, bid, nb, C, wred, nullptr, TRACE && tr ? tr + 15 : nullptr);
         if (!__syncthreads_and(ok)) goto out;  // S2
         if (C.act != kRun) break;
       }
@@ -937,9 +1022,10 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
 
     T s[P], q[P];  // direction; q: Z*res before sweep A, As after it
     unsigned hready = 0;  // halo-carrying reductions completed
+    unsigned wbits = 0;   // SP: maskT of this thread's points
 
     // ---------------------------------------------------------------- init
-    // res = forc - A sol, solve_streamfct.f90:196-201
+    // res = forc - A sol, solve_streamfct.f90:196-201 / solve_pressure.f90:163-168
     {
       double v[4] = {0.0, 0.0, 0.0, 0.0};  // beta, bb, rr, zresmax
 #pragma unroll
@@ -957,16 +1043,22 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
             rv = f - apply_point(op, g, (const T*)res_solv<T>(Pm), i, j);
             w = op.W[g.at(i, j)];
             x = res_solv<T>(Pm)[g.at(i, j)];
-            const T zr = w * rv;
-            if constexpr (WGT)
-              v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly]) * zr) * rv;
-            else
-              v[0] += (double)zr * (double)rv;
-            if (w != (T)0) {
-              v[1] += (double)f * (double)f;
-              v[2] += (double)rv * (double)rv;
+            const T zr = SP ? rv : w * rv;
+            if constexpr (SP) {  // multiplied by the weight, so a NaN on land spreads as in the reference
+              wbits |= w != (T)0 ? 1u << u : 0u;
+              v[0] += (double)rv * (double)rv * (double)w;
+              v[1] += (double)f * (double)f * (double)w;
+            } else {
+              if constexpr (WGT)
+                v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly]) * zr) * rv;
+              else
+                v[0] += (double)zr * (double)rv;
+              if (w != (T)0) {
+                v[1] += (double)f * (double)f;
+                v[2] += (double)rv * (double)rv;
+              }
+              v[3] = fmax(v[3], fabs((double)zr));
             }
-            v[3] = fmax(v[3], fabs((double)zr));
             q[u] = zr;
             stage_one(spub, pw, ph, lx, ly, zr);
             stage_one(spub + nent, pw, ph, lx, ly, (T)0);
@@ -976,7 +1068,7 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
           col_put(bx, k, x);
         }
         tm_st<CW>(t_res + c * CW, br);
-        tm_st<CW>(t_z + c * CW, bz);
+        if constexpr (!SP) tm_st<CW>(t_z + c * CW, bz);
         tm_st<CW>(t_sol + c * CW, bx);
       }
       tm_wait_st();
@@ -1030,13 +1122,20 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
               const T so = (u > 0) ? s[u > 0 ? u - 1 : 0] : ss[k - sp];
               const T fxw = sfx[ly * (pw + 1) + lx], fxe = sfx[ly * (pw + 1) + lx + 1];
               const T fyn = sfy[(ly + 1) * pw + lx];
-              const T a = axi * sbx[ly] * (fxe * (se - sc) + fxw * (sw - sc)) +
-                          sbx[ph + ly] * (fyn * (sn - sc) + fys * (so - sc));
-              if constexpr (WGT)
-                v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly]) * sc) * a;
-              else
-                v[0] += (double)sc * (double)a;
-              v[1] = fmax(v[1], fabs((double)sc));
+              T a = axi * sbx[ly] * (fxe * (se - sc) + fxw * (sw - sc)) +
+                    sbx[ph + ly] * (fyn * (sn - sc) + fys * (so - sc));
+              if constexpr (SP) {
+                const bool wet = wbits >> u & 1u;
+                a += (wet ? op.dcoef : (T)0) * sc;
+                v[0] += (double)sc * (double)a * (wet ? 1.0 : 0.0);  // a NaN on land spreads, as in the reference
+                v[1] = fmax(v[1], wet ? fabs((double)sc) : 0.0);
+              } else {
+                if constexpr (WGT)
+                  v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly]) * sc) * a;
+                else
+                  v[0] += (double)sc * (double)a;
+                v[1] = fmax(v[1], fabs((double)sc));
+              }
               q[u] = a;
               fys = fyn;
             }
@@ -1063,21 +1162,26 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
         for (int c = 0; c < NC; c++) {
           uint32_t br[CW], bz[CW];
           tm_ld<CW>(t_res + c * CW, br);
-          tm_ld<CW>(t_z + c * CW, bz);
+          if constexpr (!SP) tm_ld<CW>(t_z + c * CW, bz);
           tm_wait_ld();
 #pragma unroll
           for (int k = 0; k < CH; k++) {
             const int u = c * CH + k;
             if (u < nrow) {
-              const T w = colT_get<T>(bz, k);
               const T rv = colT_get<T>(br, k) - alpha * q[u];
-              const T zr = w * rv;
-              if constexpr (WGT)
-                v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly0 + u]) * zr) * rv;
-              else
-                v[0] += (double)zr * (double)rv;
-              if (w != (T)0) v[1] += (double)rv * (double)rv;
-              q[u] = zr;
+              if constexpr (SP) {
+                v[0] += (double)rv * (double)rv * ((wbits >> u & 1u) ? 1.0 : 0.0);
+                q[u] = rv;
+              } else {
+                const T w = colT_get<T>(bz, k);
+                const T zr = w * rv;
+                if constexpr (WGT)
+                  v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly0 + u]) * zr) * rv;
+                else
+                  v[0] += (double)zr * (double)rv;
+                if (w != (T)0) v[1] += (double)rv * (double)rv;
+                q[u] = zr;
+              }
               col_put(br, k, rv);
             }
           }
@@ -1148,7 +1252,7 @@ out:
 }
 
 // Block layout: warp 0 is the controller, warps 1-15 the workers (res_solve).
-template <int P, bool TRACE>
+template <int P, bool TRACE, bool SP>
 __global__ void __launch_bounds__(kResThreads, 1) cg_res_kernel(const __grid_constant__ CGResParams Pm) {
   extern __shared__ __align__(16) double sm[];
   __shared__ uint32_t s_tmem;
@@ -1158,7 +1262,7 @@ __global__ void __launch_bounds__(kResThreads, 1) cg_res_kernel(const __grid_con
     tc::tmem_alloc(&s_tmem, 512);
     tc::tmem_relinquish();
   }
-  res_solve<double, P, TRACE>(Pm, (int)blockIdx.x, sm, &s_tmem, C, wred);
+  res_solve<double, P, TRACE, false, false, SP>(Pm, (int)blockIdx.x, sm, &s_tmem, C, wred);
   if ((threadIdx.x >> 5) == 0) tc::tmem_dealloc(s_tmem, 512);
 }
 
@@ -1236,12 +1340,15 @@ __global__ void __launch_bounds__(kResThreads, 1) cg_res_multi_kernel(const __gr
   if ((threadIdx.x >> 5) == 0) tc::tmem_dealloc(s_tmem, 512);
 }
 
-template __global__ void cg_res_kernel<4, false>(const __grid_constant__ CGResParams);
-template __global__ void cg_res_kernel<8, false>(const __grid_constant__ CGResParams);
-template __global__ void cg_res_kernel<16, false>(const __grid_constant__ CGResParams);
-template __global__ void cg_res_kernel<4, true>(const __grid_constant__ CGResParams);
-template __global__ void cg_res_kernel<8, true>(const __grid_constant__ CGResParams);
-template __global__ void cg_res_kernel<16, true>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<4, false, false>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<8, false, false>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<16, false, false>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<4, false, true>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<8, false, true>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<16, false, true>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<4, true, false>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<8, true, false>(const __grid_constant__ CGResParams);
+template __global__ void cg_res_kernel<16, true, false>(const __grid_constant__ CGResParams);
 template __global__ void cg_res_multi_kernel<16, false>(const __grid_constant__ ResMultiParams);
 template __global__ void cg_res_multi_kernel<16, true>(const __grid_constant__ ResMultiParams);
 template __global__ void cg_res32_kernel<16>(const __grid_constant__ CGResParams);
@@ -1653,18 +1760,27 @@ const void* cg_res32_kernel_ptr(int p) {
 
 const void* cg_res_kernel_ptr(int p, bool single) {
   switch (p) {
-    case 4: return single ? (const void*)cg_res1_kernel<4> : (const void*)cg_res_kernel<4, false>;
-    case 8: return single ? (const void*)cg_res1_kernel<8> : (const void*)cg_res_kernel<8, false>;
-    case 16: return single ? (const void*)cg_res1_kernel<16> : (const void*)cg_res_kernel<16, false>;
+    case 4: return single ? (const void*)cg_res1_kernel<4> : (const void*)cg_res_kernel<4, false, false>;
+    case 8: return single ? (const void*)cg_res1_kernel<8> : (const void*)cg_res_kernel<8, false, false>;
+    case 16: return single ? (const void*)cg_res1_kernel<16> : (const void*)cg_res_kernel<16, false, false>;
+    default: return nullptr;
+  }
+}
+
+const void* cg_res_sp_kernel_ptr(int p) {
+  switch (p) {
+    case 4: return (const void*)cg_res_kernel<4, false, true>;
+    case 8: return (const void*)cg_res_kernel<8, false, true>;
+    case 16: return (const void*)cg_res_kernel<16, false, true>;
     default: return nullptr;
   }
 }
 
 const void* cg_res_trace_kernel_ptr(int p) {
   switch (p) {
-    case 4: return (const void*)cg_res_kernel<4, true>;
-    case 8: return (const void*)cg_res_kernel<8, true>;
-    case 16: return (const void*)cg_res_kernel<16, true>;
+    case 4: return (const void*)cg_res_kernel<4, true, false>;
+    case 8: return (const void*)cg_res_kernel<8, true, false>;
+    case 16: return (const void*)cg_res_kernel<16, true, false>;
     default: return nullptr;
   }
 }

@@ -101,6 +101,8 @@ __host__ __device__ constexpr int res_threads(int w, int h, int p) { return w * 
 // (the reference's recurrences) or one (single = true: A p by recurrence and
 // (p, Ap) by its exact expansion in products of the sweep before).
 const void* cg_res_kernel_ptr(int p, bool single);
+// The two-reduction kernel of congrad_surf_press (mask weights 0 or 1).
+const void* cg_res_sp_kernel_ptr(int p);
 // The two-reduction kernel with FP32 fields at p = 16 or 32 points per thread.
 const void* cg_res32_kernel_ptr(int p);
 // Dynamic shared memory of a w x h piece of the FP32 kernel: the stencil

@@ -41,6 +41,7 @@ struct pyomgpu_ctx {
   double *hur = nullptr, *hvr = nullptr, *hu = nullptr, *hv = nullptr, *mT = nullptr, *mU = nullptr, *mV = nullptr;
   OpBuf sf, sp;
   bool have_sp = false;
+  bool sp_mask01 = false;  // maskT(:,:,nz) holds only 0 and 1 (the resident kernel keeps it as bits)
   // islands
   bool have_islands = false, have_psin = false, have_line_psin = false, lu_singular = false;
   IslandSet isl;

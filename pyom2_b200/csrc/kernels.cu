@@ -120,6 +120,41 @@ __global__ void k_fill_cyclic_padded(Geo g, double* a) {
   a[g.at(i, j)] = a[g.at(si, sj)];
 }
 
+// Halo index of work item t: the rows j = -1, 0, ny+1, ny+2 whole, then the columns i = -1, 0, nx+1, nx+2 of
+// the other rows.
+__device__ __forceinline__ bool decode_halo(const Geo& g, int t, int& i, int& j) {
+  const int X = g.nx + 2 * kOnx, rows = 2 * kOnx * X;
+  if (t < rows) {
+    i = t % X - 1;
+    const int r = t / X;
+    j = r < kOnx ? r - 1 : g.ny + r - kOnx + 1;
+    return true;
+  }
+  const int u = t - rows;
+  if (u >= 2 * kOnx * g.ny) return false;
+  const int c = u % (2 * kOnx);
+  i = c < kOnx ? c - 1 : g.nx + c - kOnx + 1;
+  j = u / (2 * kOnx) + 1;
+  return true;
+}
+
+// congrad_surf_press adds alpha*p to psi over the whole array
+// (solve_pressure.f90:187), so a halo point of psi moves with its cyclic source
+// but keeps the difference it came in with.  The resident kernel updates the
+// interior; these two keep the difference and add it back.
+template <bool RESTORE>
+__global__ void k_halo_offset(Geo g, double* __restrict__ a, double* __restrict__ off) {
+  int i, j;
+  if (!decode_halo(g, (int)(blockIdx.x * blockDim.x + threadIdx.x), i, j)) return;
+  int si, sj;
+  cyclic_source(g, i, j, si, sj);
+  if (si < 1 || si > g.nx || sj < 1 || sj > g.ny) return;  // halo of a non-cyclic direction
+  if (RESTORE)
+    a[g.at(i, j)] = a[g.at(si, sj)] + off[g.at(i, j)];
+  else
+    off[g.at(i, j)] = a[g.at(i, j)] - a[g.at(si, sj)];
+}
+
 // ---------------------------------------------------------------------------
 // layout conversion
 // ---------------------------------------------------------------------------
@@ -582,6 +617,15 @@ void launch_residual_f32(const Geo& g, const OpDev<double>& op, const double* fo
 
 void launch_add_correction(const Geo& g, double* x, const float* e, double c, cudaStream_t st) {
   k_add_correction<<<std::min<size_t>(nblk((size_t)g.nx * g.ny, 256), 4096), 256, 0, st>>>(g, x, e, c);
+}
+
+void launch_halo_offset(const Geo& g, const double* a, double* off, cudaStream_t st) {
+  const int n = 2 * kOnx * (g.nx + 2 * kOnx + g.ny);
+  k_halo_offset<false><<<(n + 255) / 256, 256, 0, st>>>(g, const_cast<double*>(a), off);
+}
+void launch_halo_restore(const Geo& g, double* a, const double* off, cudaStream_t st) {
+  const int n = 2 * kOnx * (g.nx + 2 * kOnx + g.ny);
+  k_halo_offset<true><<<(n + 255) / 256, 256, 0, st>>>(g, a, const_cast<double*>(off));
 }
 
 void launch_fill_cyclic(const Geo& g, double* a, cudaStream_t st) {

@@ -33,6 +33,10 @@ void launch_unpack(const Geo& g, const double* padded, double* user, bool setcyc
 void launch_setcyclic_user(const Geo& g, double* user, cudaStream_t st);
 // setcyclic_xy on a padded field
 void launch_fill_cyclic(const Geo& g, double* padded, cudaStream_t st);
+// off = a - (the interior point setcyclic_xy copies there) at the cyclic halo positions of a, and back:
+// a = that interior point + off.
+void launch_halo_offset(const Geo& g, const double* padded, double* off, cudaStream_t st);
+void launch_halo_restore(const Geo& g, double* padded, const double* off, cudaStream_t st);
 
 // res = A p over the interior, zero halo; p and res in Fortran layout.
 void launch_apply_op_user(const Geo& g, const OpDev<double>& op, const double* p_user, double* res_user,
