@@ -159,11 +159,6 @@ double res_iter_ns(int w, int h, int p, int nb, bool f32 = false) {
 // the smallest estimated iteration time (res_iter_ns), or with
 // least_block_time the smallest iteration time x pieces.  cost: the
 // estimate.  False when none fits.
-struct ResCut {
-  int npx = 0, npy = 0, w = 0, h = 0, p = 0;
-  size_t smem = 0;
-  double cost = 1e300;
-};
 bool res_cut(int nx, int ny, int maxb, size_t cap, int p_fixed, bool least_block_time, ResCut& out,
              bool f32 = false) {
   out = ResCut{};
@@ -195,6 +190,32 @@ bool res_cut(int nx, int ny, int maxb, size_t cap, int p_fixed, bool least_block
       }
     }
   return out.npx > 0;
+}
+
+// Estimated iteration time (ns) of the cluster kernel on nb pieces of w x h
+// points with nt threads of p points, fitted to ~25 cuts each of grids from
+// 24x20 to 260x130 (1.0-4.0 us, within ~0.15): a block alone pays no remote
+// round trip; more blocks mean more slots to sum, more threads more warps to
+// reduce, and a long boundary more records.  The measured best cuts: 24x20 one
+// block 1.02 us (resident kernel 4.56), 40x40 four blocks 1.60 (4.52), 80x64
+// 1.82 (4.88), 181x91 2.64 (4.92), 260x130 3.53 (4.89); FP32 250x125 2.93 (7.4
+// to 10 us).
+double clu_iter_ns(int w, int h, int p, int nt, int nb) {
+  const double edge = 3.0 * (w + h);
+  if (nb == 1) return nt == 128 ? 860.0 + 45.0 * p : 950.0 + 85.0 * p;
+  return edge + (nt == 128 ? 1000.0 + 100.0 * p + 20.0 * nb : 1050.0 + 130.0 * p + 42.0 * nb);
+}
+
+void clu_config(const ResCut& cut, cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, cudaStream_t st) {
+  cfg.gridDim = dim3(cut.npx * cut.npy);
+  cfg.blockDim = dim3(cut.nt);
+  cfg.dynamicSmemBytes = cut.smem;
+  cfg.stream = st;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cut.npx * cut.npy;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
 }
 
 // Dynamic shared memory the resident kernels may use on this device: the
@@ -270,6 +291,126 @@ int res_plan(pyomgpu_ctx* c) {
 bool use_resident(pyomgpu_ctx* c) {
   if (c->cg_kernel == 1) return false;
   return res_plan(c) == PYOMGPU_OK && c->resd.ok;
+}
+
+// Cut of the grid for the cluster kernel (cg_clu.cu): among the cuts into at
+// most kCluMaxBlocks pieces that fit its threads and shared memory, the one
+// with the smallest estimated iteration time.  es: bytes of a field value.
+bool clu_cut(int nx, int ny, size_t cap, size_t es, ResCut& out) {
+  out = ResCut{};
+  for (int npx = 1; npx <= std::min(nx / 2, kCluMaxBlocks); npx++)
+    for (int npy = 1; npy <= ny / 2 && npx * npy <= kCluMaxBlocks; npy++) {
+      const int w = (nx + npx - 1) / npx, h = (ny + npy - 1) / npy, nb = npx * npy;
+      for (int nt : kCluNT)
+        for (int p : kCluP) {
+          const size_t bytes = clu_smem_bytes(w, h, p, es);
+          if (bytes > cap) continue;
+          if (w + h > nt || res_threads(w, h, p) > nt) continue;  // a thread receives at most two halo records
+          const double cost = clu_iter_ns(w, h, p, nt, nb);
+          if (cost < out.cost) {
+            out.npx = npx;
+            out.npy = npy;
+            out.w = w;
+            out.h = h;
+            out.p = p;
+            out.nt = nt;
+            out.smem = bytes;
+            out.cost = cost;
+          }
+        }
+    }
+  return out.npx > 0;
+}
+
+// Plans (once) the cluster kernel for this grid; R.clu[fp32].npx > 0 where it
+// fits and is estimated faster than the resident kernel's cut.
+int clu_plan(pyomgpu_ctx* c, bool fp32) {
+  auto& R = c->resd;
+  if (R.clu_planned[fp32]) return PYOMGPU_OK;
+  R.clu_planned[fp32] = true;
+  int optin = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess) return PYOMGPU_OK;
+  size_t stat = 0;
+  std::vector<const void*> ks;
+  for (int nt : kCluNT)
+    for (int p : kCluP)
+      for (bool sp : {false, true})
+        if (const void* k = cg_clu_kernel_ptr(nt, p, sp, fp32)) ks.push_back(k);
+  for (const void* k : ks) {
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return PYOMGPU_OK;
+    stat = std::max(stat, fa.sharedSizeBytes);
+  }
+  if ((size_t)optin <= stat) return PYOMGPU_OK;
+  const size_t cap = (size_t)optin - stat;
+  ResCut cut, res;
+  if (!clu_cut(c->nx, c->ny, cap, fp32 ? 4 : 8, cut)) return PYOMGPU_OK;
+  if (res_cut(c->nx, c->ny, std::min(c->nsm, kResMaxSlots - 1), res_smem_cap(c), 0, false, res, fp32) &&
+      res.cost <= cut.cost)
+    return PYOMGPU_OK;
+  for (const void* k : ks)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      return fail(PYOMGPU_ECUDA, "cannot reserve shared memory for the cluster kernel");
+  // a device or partition that cannot hold the cluster keeps the resident kernel
+  for (bool sp : {false, true}) {
+    const void* k = cg_clu_kernel_ptr(cut.nt, cut.p, sp, fp32);
+    if (!k) continue;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    clu_config(cut, cfg, at, 0);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return PYOMGPU_OK;
+    }
+  }
+  R.clu[fp32] = cut;
+  return PYOMGPU_OK;
+}
+
+// Whether the automatic choice runs this grid's solves in one cluster.
+bool use_cluster(pyomgpu_ctx* c, bool fp32) {
+  return c->cg_kernel == 0 && clu_plan(c, fp32) == PYOMGPU_OK && c->resd.clu[fp32].npx > 0;
+}
+
+int launch_cluster(pyomgpu_ctx* c, CGResParams& P, const ResCut& cut, bool surf_press, bool fp32, cudaStream_t st) {
+  P.npx = cut.npx;
+  P.npy = cut.npy;
+  P.wmax = cut.w;
+  P.hmax = cut.h;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  clu_config(cut, cfg, at, st);
+  void* args[] = {&P};
+  CK(cudaMemsetAsync(c->ctl, 0, sizeof(SyncCtl), st));
+  CK(cudaEventRecord(c->e0, st));
+  CK(cudaLaunchKernelExC(&cfg, cg_clu_kernel_ptr(cut.nt, cut.p, surf_press, fp32), args));
+  CK(cudaEventRecord(c->e1, st));
+  return 0;
+}
+
+// A small grid's solve in one cluster (cg_clu.cu).
+int run_cg_clu(pyomgpu_ctx* c, bool surf_press, const double* forc_dev, double eps, int max_it, double rtol,
+               pyomgpu_solve_info* info, cudaStream_t st) {
+  CGResParams P{};
+  P.g = c->g;
+  P.op = surf_press ? c->sp.dev() : c->sf.dev();
+  P.forc = forc_dev;
+  P.sol = c->sol;
+  P.eps = eps;
+  P.rtol = rtol;
+  P.max_it = max_it;
+  P.ctl = c->ctl;
+  P.timeout_ns = (unsigned long long)(c->timeout_s * 1e9);
+  P.stall_extra = c->stall_next;
+  c->stall_next = 0;
+  P.out = c->d_result;
+  const bool cyclic = c->g.cyclic_x || c->g.cyclic_y;
+  if (surf_press && cyclic) launch_halo_offset(c->g, c->sol, c->s0, st);
+  if (int rc = launch_cluster(c, P, c->resd.clu[0], surf_press, false, st)) return rc;
+  if (surf_press && cyclic) launch_halo_restore(c->g, c->sol, c->s0, st);
+  return finish_cg(c, info, st);
 }
 
 // The streamfunction solve (or, with surf_press, congrad_surf_press) in the
@@ -364,35 +505,39 @@ int res_plan32(pyomgpu_ctx* c) {
 int run_cg_res32(pyomgpu_ctx* c, const OpDev<float>& op, const float* b, float* x, double rtol, int max_it,
                  PipeResult* res, float* ms, cudaStream_t st) {
   auto& R = c->resd;
-  const int nb = R.npx32 * R.npy32;
-  CK(cudaMemsetAsync(c->ctl, 0, sizeof(SyncCtl), st));
-  CK(cudaMemsetAsync(R.res32, 0, c->g.size() * sizeof(float), st));
-  CK(cudaMemsetAsync(R.slots32, 0xFF, (size_t)4 * (nb + 1) * kResSlotWords * sizeof(double), st));
-  CK(cudaMemsetAsync(R.hx32, 0xFF, 2 * c->g.size() * sizeof(double), st));
   CGResParams P{};
   P.g = c->g;
   P.op32 = op;
   P.forc32 = b;
   P.sol32 = x;
-  P.res32 = R.res32;
-  P.hx = R.hx32;
-  P.hsize = (long long)c->g.size();
-  P.slots = R.slots32;
-  P.nslot = nb + 1;
-  P.npx = R.npx32;
-  P.npy = R.npy32;
-  P.wmax = R.wmax32;
-  P.hmax = R.hmax32;
   P.eps = 0.0;
   P.rtol = rtol;
   P.max_it = max_it;
   P.ctl = c->ctl;
   P.timeout_ns = (unsigned long long)(c->timeout_s * 1e9);
   P.out = c->d_result;
-  void* args[] = {&P};
-  CK(cudaEventRecord(c->e0, st));
-  CK(cudaLaunchCooperativeKernel(cg_res32_kernel_ptr(R.p32), dim3(nb), dim3(kResThreads), args, R.smem32, st));
-  CK(cudaEventRecord(c->e1, st));
+  if (use_cluster(c, true)) {
+    if (int rc = launch_cluster(c, P, R.clu[1], false, true, st)) return rc;
+  } else {
+    const int nb = R.npx32 * R.npy32;
+    CK(cudaMemsetAsync(c->ctl, 0, sizeof(SyncCtl), st));
+    CK(cudaMemsetAsync(R.res32, 0, c->g.size() * sizeof(float), st));
+    CK(cudaMemsetAsync(R.slots32, 0xFF, (size_t)4 * (nb + 1) * kResSlotWords * sizeof(double), st));
+    CK(cudaMemsetAsync(R.hx32, 0xFF, 2 * c->g.size() * sizeof(double), st));
+    P.res32 = R.res32;
+    P.hx = R.hx32;
+    P.hsize = (long long)c->g.size();
+    P.slots = R.slots32;
+    P.nslot = nb + 1;
+    P.npx = R.npx32;
+    P.npy = R.npy32;
+    P.wmax = R.wmax32;
+    P.hmax = R.hmax32;
+    void* args[] = {&P};
+    CK(cudaEventRecord(c->e0, st));
+    CK(cudaLaunchCooperativeKernel(cg_res32_kernel_ptr(R.p32), dim3(nb), dim3(kResThreads), args, R.smem32, st));
+    CK(cudaEventRecord(c->e1, st));
+  }
   CK(cudaMemcpyAsync(c->h_result, c->d_result, sizeof(CGResult), cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(c->h_scal, &c->ctl->error, sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -411,7 +556,10 @@ int run_cg_res32(pyomgpu_ctx* c, const OpDev<float>& op, const float* b, float* 
 int run_cg_ref(pyomgpu_ctx* c, bool surf_press, const double* forc_dev, double eps, int max_it, double rtol,
                pyomgpu_solve_info* info, cudaStream_t st) {
   // congrad_surf_press runs on chip too wherever the grid fits and the mask is 0/1 (1440x720: 51.2 ms tiled)
-  if ((!surf_press || c->sp_mask01) && use_resident(c))
+  const bool on_chip = !surf_press || c->sp_mask01;
+  if (on_chip && use_cluster(c, false) && c->resd.trace_nit == 0)
+    return run_cg_clu(c, surf_press, forc_dev, eps, max_it, rtol, info, st);
+  if (on_chip && use_resident(c))
     return run_cg_res(c, surf_press, forc_dev, eps, max_it, rtol, info, st);
   const OpBuf& op = surf_press ? c->sp : c->sf;
   const size_t bytes = c->g.size() * sizeof(double);

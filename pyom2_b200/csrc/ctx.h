@@ -11,6 +11,7 @@
 #include "cg_batch.cuh"
 #include "cg_pipe.cuh"
 #include "cg_ref.cuh"
+#include "cg_clu.cuh"
 #include "cg_res.cuh"
 #include "common.cuh"
 #include "islands.h"
@@ -27,6 +28,14 @@ using pyomgpu::OpBuf;
 using pyomgpu::OpDev;
 using pyomgpu::PipeResult;
 using pyomgpu::SyncCtl;
+
+// Cut of a grid into npx x npy pieces of at most w x h points, p points per
+// thread (nt threads: cluster kernel), with its dynamic shared memory and estimated iteration time (ns).
+struct ResCut {
+  int npx = 0, npy = 0, w = 0, h = 0, p = 0, nt = 0;
+  size_t smem = 0;
+  double cost = 1e300;
+};
 
 struct pyomgpu_ctx {
   int device = 0, nsm = 0;
@@ -104,6 +113,9 @@ struct pyomgpu_ctx {
     size_t smem = 0;
     double *hx = nullptr, *slots = nullptr;
     unsigned tag_gen = 0;  // generation of the next solve's epoch tags (0 .. 4094)
+    // one-cluster kernel of small grids (cg_clu.cu), FP64 and FP32 fields; npx = 0: not used
+    bool clu_planned[2] = {false, false};
+    ResCut clu[2];
     // FP32 instance (cg_res32_kernel, the mixed-precision correction solves)
     bool planned32 = false, ok32 = false;
     int npx32 = 0, npy32 = 0, wmax32 = 0, hmax32 = 0, p32 = 0;
