@@ -156,8 +156,11 @@ __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, dou
       : "=d"(d0), "=d"(d1)
       : "d"(a), "d"(b), "d"(0.0));
 }
+// mma.sync.aligned wants the warp converged: after a loop that lanes leave one by
+// one (a poll) it is not, and the instruction faults.
 __device__ __forceinline__ double warp_sum_mma(double v) {
   double d0, d1;
+  __syncwarp();
   dmma_8x8x4(d0, d1, 1.0, v);
   dmma_8x8x4(d0, d1, d0 + d1, 1.0);
   return d0;
