@@ -151,16 +151,20 @@ __device__ __forceinline__ double warp_max(double v) {
 // an 8 x 4 operand times ones give the total.  Two dependent DMMAs and an add:
 // 74 cycles (sixteen warps at once: 156) where the ten shuffles of a 64-bit
 // tree cost 183 (193).
+// mma.sync.aligned faults unless the whole warp executes it together, and after
+// divergent code (a poll that lanes leave one by one, conditional operands) it
+// may not: the warp barrier sits in the same statement, where nothing can be
+// moved in between.
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+  asm volatile(
+      "bar.warp.sync 0xffffffff;\n\t"
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
       : "=d"(d0), "=d"(d1)
-      : "d"(a), "d"(b), "d"(0.0));
+      : "d"(a), "d"(b), "d"(0.0)
+      : "memory");
 }
-// mma.sync.aligned wants the warp converged: after a loop that lanes leave one by
-// one (a poll) it is not, and the instruction faults.
 __device__ __forceinline__ double warp_sum_mma(double v) {
   double d0, d1;
-  __syncwarp();
   dmma_8x8x4(d0, d1, 1.0, v);
   dmma_8x8x4(d0, d1, d0 + d1, 1.0);
   return d0;
