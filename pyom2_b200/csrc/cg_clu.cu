@@ -383,17 +383,25 @@ __global__ void __launch_bounds__(NT, 1) cg_clu_kernel(const __grid_constant__ C
         s[u] = q[u] + bq * s[u];
         if (u < nrow) o[u * sp] = s[u];
       }
+      if (halo) {  // the whole warp polls until all its records are there (see warp_sum_mma)
+        T hq[2], hd2[2];
+        unsigned long long t0 = 0;
+        for (unsigned spin = 0;; spin++) {
+          bool ok = true;
 #pragma unroll
-      for (int e = 0; e < 2; e++)
-        if (hs[e] >= 0) {
-          T hq, hd2;
-          unsigned long long t0 = 0;
-          for (unsigned spin = 1; !dead && !clu_get(hr[e], hq, hd2, xch); spin++) {
-            if (spin == 1) t0 = globaltimer_ns();
-            if (clu_expired(R.err, spin, t0, R.tmo)) dead = true;
+          for (int e = 0; e < 2; e++)
+            if (hs[e] >= 0) ok = clu_get(hr[e], hq[e], hd2[e], xch) && ok;
+          if (__all_sync(0xffffffffu, ok)) break;
+          if (spin == 0) t0 = globaltimer_ns();
+          if (__any_sync(0xffffffffu, clu_expired(R.err, spin + 1, t0, R.tmo))) {
+            dead = true;
+            break;
           }
-          if (!dead) ss[hs[e]] = hq + bq * hd2;
         }
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+          if (hs[e] >= 0 && !dead) ss[hs[e]] = hq[e] + bq * hd2[e];
+      }
       xch++;
     }
     if (!block_sync()) goto out;

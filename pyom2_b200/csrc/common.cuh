@@ -150,22 +150,22 @@ __device__ __forceinline__ double warp_max(double v) {
 // operand times ones give eight column sums, two of them in a lane; their sums as
 // an 8 x 4 operand times ones give the total.  Two dependent DMMAs and an add:
 // 74 cycles (sixteen warps at once: 156) where the ten shuffles of a 64-bit
-// tree cost 183 (193).
-// mma.sync.aligned faults unless the whole warp executes it together, and after
-// divergent code (a poll that lanes leave one by one, conditional operands) it
-// may not: the warp barrier sits in the same statement, where nothing can be
-// moved in between.
+// tree cost 183 (193).  One-dimensional blocks only (the lane is threadIdx.x).
+// mma.sync.aligned faults unless the whole warp executes it together.  After a
+// loop that lanes leave one by one (a poll) they stay apart, and a warp barrier
+// before the mma did not help: .aligned lets the compiler take convergence for
+// granted and drop it.  So the operand first passes through a shuffle, which
+// brings the lanes together and cannot be dropped.
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
-  asm volatile(
-      "bar.warp.sync 0xffffffff;\n\t"
-      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
-      : "=d"(d0), "=d"(d1)
-      : "d"(a), "d"(b), "d"(0.0)
-      : "memory");
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+               : "=d"(d0), "=d"(d1)
+               : "d"(a), "d"(b), "d"(0.0)
+               : "memory");
 }
 __device__ __forceinline__ double warp_sum_mma(double v) {
+  const int lo = __shfl_sync(0xffffffffu, __double2loint(v), (int)threadIdx.x & 31);
   double d0, d1;
-  dmma_8x8x4(d0, d1, 1.0, v);
+  dmma_8x8x4(d0, d1, 1.0, __hiloint2double(__double2hiint(v), lo));
   dmma_8x8x4(d0, d1, d0 + d1, 1.0);
   return d0;
 }
