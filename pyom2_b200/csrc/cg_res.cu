@@ -309,7 +309,7 @@ __device__ void ctl1_iter(ResCtl& C, const CGResParams& P, const double* v) {
 template <typename T>
 struct HaloT {
   int sidx;       // shared-memory index (-1: none)
-  long long gidx; // padded position whose exchange record is received
+  int gidx;       // padded position whose exchange record is received
   T q, s;         // received Z*res and direction
 };
 using Halo = HaloT<double>;
@@ -324,15 +324,14 @@ __device__ __forceinline__ bool worker_halo_load_tagged(const CGResParams& P, Ha
   int* const err = &P.ctl->error;
   const unsigned long long tmo = P.timeout_ns;
   const unsigned long long t0 = globaltimer_ns();
-  // one record after the other (a worker rarely has two)
-#pragma unroll 1
-  for (int e = 0; e < 2; e++) {
+#pragma unroll
+  for (int e = 0; e < 2; e++) {  // unrolled: an index would move the records to local memory
     if (hl[e].sidx < 0) continue;
     for (unsigned spin = 1;; spin++) {
       bool ok;
       if constexpr (sizeof(T) == 8) {
         unsigned long long w0, w1, w2, w3;
-        ld_relaxed_v4_u64(hx + 4 * hl[e].gidx, w0, w1, w2, w3);
+        ld_relaxed_v4_u64(hx + 4 * (size_t)hl[e].gidx, w0, w1, w2, w3);
         ok = tag_ok(w0, tag) && tag_ok(w1, tag) && tag_ok(w2, tag) && tag_ok(w3, tag);
         if (ok) {
           hl[e].q = untag(w0, w1);
@@ -340,7 +339,7 @@ __device__ __forceinline__ bool worker_halo_load_tagged(const CGResParams& P, Ha
         }
       } else {
         unsigned long long w0, w1;
-        ld_relaxed_v2_u64(hx + 2 * hl[e].gidx, w0, w1);
+        ld_relaxed_v2_u64(hx + 2 * (size_t)hl[e].gidx, w0, w1);
         ok = tag_ok(w0, tag) && tag_ok(w1, tag);
         if (ok) {
           hl[e].q = __uint_as_float((unsigned)w0);
@@ -367,6 +366,39 @@ __device__ __forceinline__ void stage_one(T* spub, int pw, int ph, int lx, int l
   if (lx == pw - 1) spub[ph + ly] = v;
   if (ly == 0) spub[2 * ph + lx] = v;
   if (ly == ph - 1) spub[2 * ph + pw + lx] = v;
+}
+
+// Both quantities of a thread's column segment (rows ly0 .. ly0+nrow-1 of column lx): the west and east tests
+// once per thread, one row each for south and north.  (stage_one on every point cost ~200 instructions a
+// thread and sweep.)
+template <typename T, int P>
+__device__ __forceinline__ void stage_segment(T* spub, int pw, int ph, int lx, int ly0, int nrow, const T (&q)[P],
+                                              const T (&s)[P]) {
+  if (nrow <= 0) return;
+  const int nent = 2 * (pw + ph);
+  if (lx == 0 || lx == pw - 1) {  // pieces are at least two columns wide
+    T* a = spub + (lx == 0 ? 0 : ph) + ly0;
+#pragma unroll
+    for (int u = 0; u < P; u++)
+      if (u < nrow) {
+        a[u] = q[u];
+        a[nent + u] = s[u];
+      }
+  }
+  if (ly0 == 0) {
+    spub[2 * ph + lx] = q[0];
+    spub[nent + 2 * ph + lx] = s[0];
+  }
+  if (ly0 + nrow == ph) {
+    T ql = q[0], sl = s[0];  // the last row's, by selects (an index would move q and s to local memory)
+#pragma unroll
+    for (int u = 1; u < P; u++) {
+      ql = u < nrow ? q[u] : ql;
+      sl = u < nrow ? s[u] : sl;
+    }
+    spub[2 * ph + pw + lx] = ql;
+    spub[nent + 2 * ph + pw + lx] = sl;
+  }
 }
 
 // The staged boundary values (NQ quantities) to the exchange records (word k
@@ -461,15 +493,33 @@ __device__ __forceinline__ double* res_slot(const CGResParams& P, unsigned ep, i
   return P.slots + ((size_t)(ep % 3u) * P.nslot + b) * kResSlotWords;
 }
 
+// Warp totals of NV values in every lane (sums; slot kMaxSlot a maximum of
+// absolute values), two sums at a time.
+template <int NV, int kMaxSlot, int K = 0>
+__device__ __forceinline__ void warp_totals(const double (&v)[NV], double (&t)[NV]) {
+  if constexpr (K < NV) {
+    if constexpr (K == kMaxSlot) {
+      t[K] = warp_max_nonneg(v[K]);
+      warp_totals<NV, kMaxSlot, K + 1>(v, t);
+    } else if constexpr (K + 1 < NV && K + 1 != kMaxSlot) {
+      warp_sum2(v[K], v[K + 1], t[K], t[K + 1]);
+      warp_totals<NV, kMaxSlot, K + 2>(v, t);
+    } else {
+      t[K] = warp_sum(v[K]);
+      warp_totals<NV, kMaxSlot, K + 1>(v, t);
+    }
+  }
+}
+
 // Worker side of a reduction: per-warp partials of the worker warps into wred.
 template <int NV, int kMaxSlot>
 __device__ __forceinline__ void worker_partials(const double (&v)[NV], double (*wred)[kResSlotWords]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double r[NV];
+  warp_totals<NV, kMaxSlot>(v, r);
 #pragma unroll
-  for (int k = 0; k < NV; k++) {
-    const double r = (k == kMaxSlot) ? warp_max(v[k]) : warp_sum(v[k]);
-    if (lane == 0) wred[w][k] = r;
-  }
+  for (int k = 0; k < NV; k++)
+    if (lane == 0) wred[w][k] = r[k];
 }
 
 // Controller side of epoch ep (warp 0, after the workers' partials are in
@@ -505,12 +555,10 @@ __device__ __forceinline__ bool controller_epoch(const CGResParams& P, unsigned 
     return slot_base + ((size_t)(e & 1u) * nslot + b) * (2 * kResSlotWords);
   };
   if constexpr (TAG) {
-    double t[NV];
+    double t[NV], x[NV];
 #pragma unroll
-    for (int k = 0; k < NV; k++) {
-      const double x = (lane >= 1 && lane < kResThreads / 32) ? wred[lane][k] : 0.0;
-      t[k] = (k == kMaxSlot) ? warp_max(x) : warp_sum(x);
-    }
+    for (int k = 0; k < NV; k++) x[k] = (lane >= 1 && lane < kResThreads / 32) ? wred[lane][k] : 0.0;
+    warp_totals<NV, kMaxSlot>(x, t);
     double mv = 0.0;
 #pragma unroll
     for (int k = 0; k < NV; k++)
@@ -642,15 +690,16 @@ __device__ __forceinline__ bool controller_epoch(const CGResParams& P, unsigned 
     __syncwarp();
     if (lane < kResSlotWords) st_weak_f64(res_slot(P, ep + 2, bid) + lane, empty_word());
   }
-  double out[NV];
+  double out[NV], sum[NV];
 #pragma unroll
   for (int k = 0; k < NV; k++) {
     double a = 0.0;
 #pragma unroll
     for (int m = 0; m < kPer; m++)
       if (have >> m & 1u) a = (k == kMaxSlot) ? fmax(a, got[m][k]) : a + got[m][k];
-    out[k] = (k == kMaxSlot) ? warp_max(a) : warp_sum(a);
+    sum[k] = a;
   }
+  warp_totals<NV, kMaxSlot>(sum, out);
   if (lane == 0) {
     if (kStep == kStepInit)
       ctl_init(C, P, out);
@@ -829,7 +878,7 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
           hy = ph;
         }
         hl[e].sidx = (hy + 1) * sp + hx + 1;
-        hl[e].gidx = (long long)g.at(ilo + hx, jlo + hy);
+        hl[e].gidx = (int)g.at(ilo + hx, jlo + hy);
       }
     }
 
@@ -904,12 +953,12 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
       {
         const int sp = opaque(pw + 2);
         const T bq = (T)C.bq;
+T* o = ss + (ly0 + 1) * sp + lx + 1;
 #pragma unroll
-        for (int u = 0; u < P; u++)
-          if (u < nrow) {
-            s[u] = q[u] + bq * s[u];
-            ss[(ly0 + u + 1) * sp + lx + 1] = s[u];
-          }
+        for (int u = 0; u < P; u++) {
+          s[u] = q[u] + bq * s[u];
+          if (u < nrow) o[u * sp] = s[u];
+        }
 #pragma unroll
         for (int e = 0; e < 2; e++)
           if (hl[e].sidx >= 0) ss[hl[e].sidx] = hl[e].q + bq * hl[e].s;
@@ -923,35 +972,37 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
         const int pw = opaque(pw_), sp = pw + 2, ph = opaque(ph_);
         double v[2] = {0.0, 0.0};  // (s, As), max|s|
         if (nrow > 0) {
-          T fys = sfy[ly0 * pw + lx];
+          // No branch per point: with one, a point's loads and its chain of a dozen FP64 operations ran before
+          // the next point's began.  Rows past the segment repeat its last one and are dropped from the sums.
+          const T *o = ss + (ly0 + 1) * sp + lx + 1, *fx = sfx + ly0 * (pw + 1) + lx, *fy = sfy + (ly0 + 1) * pw + lx;
+          const T *bx = sbx + ly0, *by = sbx + ph + ly0;
+          const T below = o[-sp], above = o[nrow * sp];
+          T fys = fy[-pw];
 #pragma unroll
-          for (int u = 0; u < P; u++)
-            if (u < nrow) {
-              const int ly = ly0 + u;
-              const int k = (ly + 1) * sp + lx + 1;
-              const T sc = s[u];
-              const T se = ss[k + 1], sw = ss[k - 1];
-              const T sn = (u + 1 < P && u + 1 < nrow) ? s[u + 1 < P ? u + 1 : u] : ss[k + sp];
-              const T so = (u > 0) ? s[u > 0 ? u - 1 : 0] : ss[k - sp];
-              const T fxw = sfx[ly * (pw + 1) + lx], fxe = sfx[ly * (pw + 1) + lx + 1];
-              const T fyn = sfy[(ly + 1) * pw + lx];
-              T a = axi * sbx[ly] * (fxe * (se - sc) + fxw * (sw - sc)) +
-                    sbx[ph + ly] * (fyn * (sn - sc) + fys * (so - sc));
-              if constexpr (SP) {
-                const bool wet = wbits >> u & 1u;
-                a += (wet ? op.dcoef : (T)0) * sc;
-                v[0] += (double)sc * (double)a * (wet ? 1.0 : 0.0);  // a NaN on land spreads, as in the reference
-                v[1] = fmax(v[1], wet ? fabs((double)sc) : 0.0);
-              } else {
-                if constexpr (WGT)
-                  v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly]) * sc) * a;
-                else
-                  v[0] += (double)sc * (double)a;
-                v[1] = fmax(v[1], fabs((double)sc));
-              }
-              q[u] = a;
-              fys = fyn;
+          for (int u = 0; u < P; u++) {
+            const int w = u == 0 ? 0 : min(u, nrow - 1);
+            const T sc = s[u];
+            const T se = o[w * sp + 1], sw = o[w * sp - 1];
+            const T sn = u + 1 == nrow ? above : s[u + 1 < P ? u + 1 : u];
+            const T so = (u > 0) ? s[u > 0 ? u - 1 : 0] : below;
+            const T fxw = fx[w * (pw + 1)], fxe = fx[w * (pw + 1) + 1];
+            const T fyn = fy[w * pw];
+            T a = axi * bx[w] * (fxe * (se - sc) + fxw * (sw - sc)) + by[w] * (fyn * (sn - sc) + fys * (so - sc));
+            if constexpr (SP) {
+              const bool wet = wbits >> u & 1u;
+              a += (wet ? op.dcoef : (T)0) * sc;
+              v[0] += u < nrow ? (double)sc * (double)a * (wet ? 1.0 : 0.0) : 0.0;  // a NaN on land spreads
+              v[1] = fmax(v[1], wet ? fabs((double)sc) : 0.0);
+            } else {
+              if constexpr (WGT)
+                v[0] += u < nrow ? (1.0 / ((double)axi * (double)by[w]) * sc) * a : 0.0;
+              else
+                v[0] += u < nrow ? (double)sc * (double)a : 0.0;
+              v[1] = fmax(v[1], u < nrow ? fabs((double)sc) : 0.0);
             }
+            q[u] = a;
+            fys = fyn;
+          }
         }
         worker_partials<2, 1>(v, wred);
       }
@@ -980,33 +1031,26 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
 #pragma unroll
           for (int k = 0; k < CH; k++) {
             const int u = c * CH + k;
-            if (u < nrow) {
-              const T rv = colT_get<T>(br, k) - alpha * q[u];
-              if constexpr (SP) {
-                v[0] += (double)rv * (double)rv * ((wbits >> u & 1u) ? 1.0 : 0.0);
-                q[u] = rv;
-              } else {
-                const T w = colT_get<T>(bz, k);
-                const T zr = w * rv;
-                if constexpr (WGT)
-                  v[0] += (1.0 / ((double)axi * (double)sbx[ph + ly0 + u]) * zr) * rv;
-                else
-                  v[0] += (double)zr * (double)rv;
-                if (w != (T)0) v[1] += (double)rv * (double)rv;
-                q[u] = zr;
-              }
-              col_put(br, k, rv);
+            const T rv = colT_get<T>(br, k) - alpha * q[u];
+            if constexpr (SP) {
+              v[0] += u < nrow ? (double)rv * (double)rv * ((wbits >> u & 1u) ? 1.0 : 0.0) : 0.0;
+              q[u] = rv;
+            } else {
+              const T w = colT_get<T>(bz, k);
+              const T zr = w * rv;
+              if constexpr (WGT)
+                v[0] += u < nrow ? (1.0 / ((double)axi * (double)sbx[ph + ly0 + u]) * zr) * rv : 0.0;
+              else
+                v[0] += u < nrow ? (double)zr * (double)rv : 0.0;
+              v[1] += w != (T)0 ? (double)rv * (double)rv : 0.0;
+              q[u] = zr;
             }
+            col_put(br, k, rv);
           }
           tm_st<CW>(t_res + c * CW, br);
         }
         // boundary points to the neighbours: (Z res, s) for their next direction
-#pragma unroll
-        for (int u = 0; u < P; u++)
-          if (u < nrow) {
-            stage_one(spub, pw, ph, lx, ly0 + u, q[u]);
-            stage_one(spub + 2 * (pw + ph), pw, ph, lx, ly0 + u, s[u]);
-          }
+        stage_segment<T, P>(spub, pw, ph, lx, ly0, nrow, q, s);
         if (TRACE && tr) tr[5] = globaltimer_ns();
         workers_sync();
         copy_out_tagged(Pm, spub, ilo, ihi, jlo, jhi, wt, res_tag(Pm, 2u * hready));
@@ -1025,7 +1069,7 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
 #pragma unroll
           for (int k = 0; k < CH; k++) {
             const int u = c * CH + k;
-            if (u < nrow) col_put(bx, k, colT_get<T>(bx, k) + alpha * s[u]);
+            col_put(bx, k, colT_get<T>(bx, k) + alpha * s[u]);
           }
           tm_st<CW>(t_sol + c * CW, bx);
         }
