@@ -63,6 +63,12 @@ struct ConvSpec {
 int conv3x3_launch(const ConvSpec& s, int nsm, cudaStream_t st);
 bool conv3x3_supported(int cin, int cout);
 
+// Weight and bias gradients of one layer (conv_dw.cu), added to dW
+// [Cout][Cin][3][3] and db [Cout]: X its planar input, G the planar gradient of
+// its output.  Same return values as conv3x3_launch.
+int conv3x3_dw_launch(int cin, int cout, const uint16_t* X, const uint16_t* G, int H, int W, float* dW, float* db,
+                      int nsm, int* err, unsigned long long timeout_ns, cudaStream_t st);
+
 // Packs f32 weights [Cout][Cin][3][3] into [tap][Cin/8][Cout][8] bf16 (round
 // to nearest even).  flip packs the backward-data kernel instead: channels
 // transposed and taps rotated by 180 degrees (its input channels are the

@@ -3,8 +3,8 @@
 // Forward and backward-data convolutions run on the tensor cores
 // (conv_tc.cu; the backward-data pass is the same kernel with the flipped
 // weight packing and the ReLU derivative fused as its gate).  The weight
-// gradient is a CUDA-core reduction over pixels (k_conv_dw), and the
-// pooling / upsampling adjoints are elementwise kernels.
+// gradient is a contraction over pixels (conv_dw.cu), and the pooling /
+// upsampling adjoints are elementwise kernels.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -44,7 +44,6 @@ size_t unet_num_params() { return unet_bias_offset(kUNetLayers); }
 
 namespace {
 
-__device__ __forceinline__ float bfv(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 __device__ __forceinline__ uint16_t tobf(float f) {
   __nv_bfloat16 h = __float2bfloat16_rn(f);
   return *reinterpret_cast<uint16_t*>(&h);
@@ -110,90 +109,6 @@ __global__ void k_pool_bwd_gate(const uint16_t* __restrict__ gdec, const uint16_
     }
     reinterpret_cast<uint4*>(out)[e] = make_uint4(o[0], o[1], o[2], o[3]);
   }
-}
-
-// ---------------------------------------------------------------- weight gradient
-// dW[co][ci][tap] += sum_p G[co][p] X[ci][p + tap - (1,1)], db[co] += sum_p G[co][p].
-// A CTA owns 16 output channels (blockIdx.y) and walks pixel tiles of 4 x 32;
-// thread (co_l, slot) accumulates the (ci, tap) pairs slot, slot+16, ...
-constexpr int kDwRows = 4, kDwCols = 32, kDwThreads = 256;
-
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kDwThreads) k_conv_dw(const uint16_t* __restrict__ X, const uint16_t* __restrict__ G,
-                                                        int H, int Wd, float* __restrict__ dW, float* __restrict__ db) {
-  constexpr int NACC = CIN * 9 / 16;
-  constexpr int SR = kDwRows + 2, SC = kDwCols + 2;
-  __shared__ uint16_t sx[CIN * SR * SC];
-  __shared__ float sg[16 * kDwRows * kDwCols];
-  const int tid = threadIdx.x, co_l = tid >> 4, slot = tid & 15;
-  const int co = blockIdx.y * 16 + co_l;
-  int off[NACC];
-  float acc[NACC];
-#pragma unroll
-  for (int k = 0; k < NACC; k++) {
-    const int q = slot + 16 * k, ci = q / 9, tap = q - 9 * ci;
-    off[k] = ci * SR * SC + (tap / 3) * SC + (tap % 3);
-    acc[k] = 0.f;
-  }
-  float accb = 0.f;
-  const int tiles_x = (Wd + kDwCols - 1) / kDwCols, tiles_y = (H + kDwRows - 1) / kDwRows;
-  const int ntiles = tiles_x * tiles_y;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int y0 = (t / tiles_x) * kDwRows, x0 = (t % tiles_x) * kDwCols;
-    __syncthreads();
-    for (int e = tid; e < CIN * SR * SC; e += kDwThreads) {
-      const int ci = e / (SR * SC), rem = e - ci * SR * SC, r = rem / SC, c = rem - r * SC;
-      const int y = y0 - 1 + r, x = x0 - 1 + c;
-      uint16_t v = 0;
-      if (y >= 0 && y < H && x >= 0 && x < Wd) v = X[(((size_t)(ci >> 3) * H + y) * Wd + x) * 8 + (ci & 7)];
-      sx[e] = v;
-    }
-    for (int e = tid; e < 16 * kDwRows * kDwCols; e += kDwThreads) {
-      const int c16 = e / (kDwRows * kDwCols), rem = e - c16 * kDwRows * kDwCols;
-      const int r = rem / kDwCols, c = rem - r * kDwCols;
-      const int y = y0 + r, x = x0 + c, cc = blockIdx.y * 16 + c16;
-      float v = 0.f;
-      if (y < H && x < Wd) v = bfv(G[(((size_t)(cc >> 3) * H + y) * Wd + x) * 8 + (cc & 7)]);
-      sg[e] = v;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int p = 0; p < kDwRows * kDwCols; p++) {
-      const int r = p / kDwCols, c = p - r * kDwCols;
-      const float g = sg[co_l * kDwRows * kDwCols + p];
-      const int base = r * SC + c;
-      accb += g;
-#pragma unroll
-      for (int k = 0; k < NACC; k++) acc[k] += g * bfv(sx[off[k] + base]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < NACC; k++) {
-    const int q = slot + 16 * k, ci = q / 9, tap = q - 9 * ci;
-    atomicAdd(&dW[((size_t)co * CIN + ci) * 9 + tap], acc[k]);
-  }
-  if (slot == 0) atomicAdd(&db[co], accb);
-}
-
-template <int CIN, int COUT>
-void launch_dw_t(const uint16_t* X, const uint16_t* G, int H, int W, float* dW, float* db, int nsm, cudaStream_t st) {
-  const int ntiles = ((W + kDwCols - 1) / kDwCols) * ((H + kDwRows - 1) / kDwRows);
-  const int gx = std::max(1, std::min(ntiles, 2 * nsm));
-  k_conv_dw<CIN, COUT><<<dim3(gx, COUT / 16), kDwThreads, 0, st>>>(X, G, H, W, dW, db);
-}
-
-void launch_dw(int cin, int cout, const uint16_t* X, const uint16_t* G, int H, int W, float* dW, float* db, int nsm,
-               cudaStream_t st) {
-#define PYOMGPU_DW_CASE(a, b) \
-  if (cin == a && cout == b) return launch_dw_t<a, b>(X, G, H, W, dW, db, nsm, st);
-  PYOMGPU_DW_CASE(16, 16)
-  PYOMGPU_DW_CASE(16, 32)
-  PYOMGPU_DW_CASE(32, 32)
-  PYOMGPU_DW_CASE(32, 64)
-  PYOMGPU_DW_CASE(64, 64)
-  PYOMGPU_DW_CASE(64, 32)
-  PYOMGPU_DW_CASE(32, 16)
-#undef PYOMGPU_DW_CASE
 }
 
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -314,9 +229,10 @@ int conv_bwd(UNet& n, int l, const uint16_t* g, uint16_t* y, const uint16_t* gat
   s.timeout_ns = n.timeout_ns;
   return conv3x3_launch(s, n.nsm, st);
 }
-void dw(UNet& n, int l, const uint16_t* x, const uint16_t* g, cudaStream_t st) {
-  launch_dw(kUNet[l].cin, kUNet[l].cout, x, g, n.H >> kUNet[l].level, n.W >> kUNet[l].level,
-            n.grads + unet_weight_offset(l), n.grads + unet_bias_offset(l), n.nsm, st);
+int dw(UNet& n, int l, const uint16_t* x, const uint16_t* g, cudaStream_t st) {
+  return conv3x3_dw_launch(kUNet[l].cin, kUNet[l].cout, x, g, n.H >> kUNet[l].level, n.W >> kUNet[l].level,
+                           n.grads + unet_weight_offset(l), n.grads + unet_bias_offset(l), n.nsm, n.err,
+                           n.timeout_ns, st);
 }
 void up_bwd(UNet& n, const uint16_t* fine, int C, int coarse_level, uint16_t* coarse, cudaStream_t st) {
   const int h = n.H >> coarse_level, w = n.W >> coarse_level;
@@ -355,37 +271,37 @@ int unet_backward(UNet& n, const float* gz, cudaStream_t st) {
   const size_t p0 = (size_t)n.H * n.W;
   k_gz_planar<<<grid_for(p0), 256, 0, st>>>(gz, p0, n.gO);
   // output layer and decoder
-  dw(n, 11, n.U1, n.gO, st);
+  if ((rc = dw(n, 11, n.U1, n.gO, st))) return rc;
   if ((rc = conv_bwd(n, 11, n.gO, n.gU1, n.U1, st))) return rc;
   up_bwd(n, n.gU1, 16, 1, n.gv10, st);
-  dw(n, 10, n.U2, n.gv10, st);
+  if ((rc = dw(n, 10, n.U2, n.gv10, st))) return rc;
   if ((rc = conv_bwd(n, 10, n.gv10, n.gU2, n.U2, st))) return rc;
   up_bwd(n, n.gU2, 32, 2, n.gv9, st);
-  dw(n, 9, n.U3, n.gv9, st);
+  if ((rc = dw(n, 9, n.U3, n.gv9, st))) return rc;
   if ((rc = conv_bwd(n, 9, n.gv9, n.gU3, n.U3, st))) return rc;
   up_bwd(n, n.gU3, 64, 3, n.gv8, st);
-  dw(n, 8, n.B4, n.gv8, st);
+  if ((rc = dw(n, 8, n.B4, n.gv8, st))) return rc;
   if ((rc = conv_bwd(n, 8, n.gv8, n.gB4, n.B4, st))) return rc;
   // bottom level
-  dw(n, 7, n.A4, n.gB4, st);
+  if ((rc = dw(n, 7, n.A4, n.gB4, st))) return rc;
   if ((rc = conv_bwd(n, 7, n.gB4, n.gA4, n.A4, st))) return rc;
-  dw(n, 6, n.P3, n.gA4, st);
+  if ((rc = dw(n, 6, n.P3, n.gA4, st))) return rc;
   if ((rc = conv_bwd(n, 6, n.gA4, n.gP3, nullptr, st))) return rc;
   // encoder, level 3 .. 1: S feeds the pool and the decoder skip
   pool_bwd(n, n.gU3, n.gP3, n.S3, 64, 2, n.gS3, st);
-  dw(n, 5, n.A3, n.gS3, st);
+  if ((rc = dw(n, 5, n.A3, n.gS3, st))) return rc;
   if ((rc = conv_bwd(n, 5, n.gS3, n.gA3, n.A3, st))) return rc;
-  dw(n, 4, n.P2, n.gA3, st);
+  if ((rc = dw(n, 4, n.P2, n.gA3, st))) return rc;
   if ((rc = conv_bwd(n, 4, n.gA3, n.gP2, nullptr, st))) return rc;
   pool_bwd(n, n.gU2, n.gP2, n.S2, 32, 1, n.gS2, st);
-  dw(n, 3, n.A2, n.gS2, st);
+  if ((rc = dw(n, 3, n.A2, n.gS2, st))) return rc;
   if ((rc = conv_bwd(n, 3, n.gS2, n.gA2, n.A2, st))) return rc;
-  dw(n, 2, n.P1, n.gA2, st);
+  if ((rc = dw(n, 2, n.P1, n.gA2, st))) return rc;
   if ((rc = conv_bwd(n, 2, n.gA2, n.gP1, nullptr, st))) return rc;
   pool_bwd(n, n.gU1, n.gP1, n.S1, 16, 0, n.gS1, st);
-  dw(n, 1, n.A1, n.gS1, st);
+  if ((rc = dw(n, 1, n.A1, n.gS1, st))) return rc;
   if ((rc = conv_bwd(n, 1, n.gS1, n.gA1, n.A1, st))) return rc;
-  dw(n, 0, n.X0, n.gA1, st);
+  if ((rc = dw(n, 0, n.X0, n.gA1, st))) return rc;
   return (int)cudaGetLastError();
 }
 
