@@ -1,7 +1,7 @@
 // tcgen05 implicit-GEMM 3x3 convolution (declarations in conv_tc.cuh).
 //
-// One CTA (8 warps) walks output tiles of ROWS rows x 128 pixels.  Per tile
-// one TMA load brings the (ROWS+2) x 130 x Cin input box (zero-filled outside
+// One CTA (8 warps) walks output tiles of ROWS rows x 126 pixels.  Per tile
+// one TMA load brings the (ROWS+2) x 128 x Cin input box (zero-filled outside
 // the image = the convolution's zero padding) into shared memory; thread 0
 // issues 9 taps x Cin/16 MMAs of M=128, N=Cout, K=16 per output row, each A
 // operand being the box shifted by the tap offset; the accumulators
@@ -33,6 +33,7 @@ namespace pyomgpu {
 namespace {
 
 constexpr int kBW = kConvTileX + 2;  // box columns
+static_assert(kBW == 128, "M rows of the MMA, and the largest TMA box row in 64-bit words");
 
 __host__ __device__ constexpr uint32_t pow2_cols(uint32_t n) {
   uint32_t c = 32;
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
   auto issue_tile = [&](int tile, int b) {
     const int ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
     mbar_arrive_expect_tx(&bar_ld[b], S::XBYTES);
-    tma_load_4d(base + b * S::XSTRIDE, &a.map_x, 0, tx * kConvTileX - 1, ty * ROWS - 1, 0, &bar_ld[b]);
+    tma_load_3d(base + b * S::XSTRIDE, &a.map_x, 2 * (tx * kConvTileX - 1), ty * ROWS - 1, 0, &bar_ld[b]);
   };
   if (tid == 0) {
     mbar_arrive_expect_tx(bar_w, S::WBYTES);
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
 
     // ---- epilogue: lane = output pixel x0 + 32*quarter + lane, channels [half*CW, (half+1)*CW)
     const int x = x0 + 32 * quarter + lane;
-    const bool in_x = x < a.W;
+    const bool in_x = 32 * quarter + lane < kConvTileX && x < a.W;  // the last two rows of M are the rim's
     const uint32_t trow = tmem + ((uint32_t)(32 * quarter) << 16);
 #pragma unroll 1
     for (int t = 0; t < ROWS; t += 2) {
@@ -344,10 +345,13 @@ int launch_one(const ConvSpec& s, int nsm, cudaStream_t st) {
     attr = true;
   }
   ConvArgs a{};
-  const uint64_t dims[4] = {8, (uint64_t)s.W, (uint64_t)s.H, (uint64_t)(CIN / 8)};
-  const uint64_t strides[3] = {16, (uint64_t)s.W * 16, (uint64_t)s.W * s.H * 16};
-  const uint32_t box[4] = {8, (uint32_t)kBW, (uint32_t)S::BH, (uint32_t)(CIN / 8)};
-  if (encode_map(&a.map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, s.x, dims, strides, box)) return -2;
+  // A row of pixels (8 bf16 channels, 16 bytes each) as 2 W 64-bit words, so that a box row is one contiguous run
+  // of 256 words (the largest box extent, hence 128 pixels).  With the 16-byte pixel as a dimension of its own
+  // the copy moved pixel by pixel: a learned solve at 720x360 took 103 ms, 95 ms this way.
+  const uint64_t dims[3] = {2 * (uint64_t)s.W, (uint64_t)s.H, (uint64_t)(CIN / 8)};
+  const uint64_t strides[2] = {(uint64_t)s.W * 16, (uint64_t)s.W * s.H * 16};
+  const uint32_t box[3] = {2 * (uint32_t)kBW, (uint32_t)S::BH, (uint32_t)(CIN / 8)};
+  if (encode_map(&a.map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, s.x, dims, strides, box)) return -2;
   a.wpack = s.wpack;
   a.bias = s.bias;
   a.y = s.y;

@@ -18,7 +18,7 @@
 
 namespace pyomgpu {
 
-constexpr int kConvTileX = 128;   // output pixels per row tile (MMA M)
+constexpr int kConvTileX = 126;  // output pixels of a tile row: a box row of 128, less its rim (conv_tc.cu)
 constexpr int kConvThreads = 256;  // 2 warpgroups: TMEM lane quarter = warp % 4, channel half = warp / 4
 
 // Epilogue of one convolution: v = acc + bias, then
@@ -31,7 +31,7 @@ constexpr int kConvThreads = 256;  // 2 warpgroups: TMEM lane quarter = warp % 4
 enum ConvEpilogue : int { kEpiPlain = 0, kEpiUp = 1, kEpiF32 = 2 };
 
 struct ConvArgs {
-  CUtensorMap map_x;      // input, box (8, 130, rows+2, Cin/8), rows = the instantiation's tile height
+  CUtensorMap map_x;      // input, box (2 x 128 64-bit words, rows+2, Cin/8), rows = the instantiation's tile height
   const uint16_t* wpack;  // [9][Cin/8][Cout][8] bf16
   const float* bias;      // [Cout] or null
   void* y;
