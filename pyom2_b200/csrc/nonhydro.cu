@@ -227,111 +227,6 @@ __device__ __forceinline__ bool nh_sweep(const NHParams& P, int cur, double bq, 
   return __syncthreads_and(ok && prod_ok) != 0;  // also: every stage is read to the end before the next sweep
 }
 
-// Scalar state of congrad_non_hydro's loop (non_hydrostatic.f90:177-242),
-// the same in every thread of every block.  The convergence test of
-// iteration n needs max|p| of the direction formed after it, so it runs after
-// the next iteration's first sweep (after_a).
-struct NHCtl {
-  enum { kGo = 0, kOk = 1, kErr = 2 };
-  double beta = 0, bb = 0, rtol2bb = 0, eps = 0, rtol = 0;
-  double betamin = 0, step1 = 0, est = 0, bq = 0, alpha_prev = 0, rr_prev = 0;
-  int max_it = 0, n = 0, status = PYOMGPU_OK;
-
-  __device__ int start(double rsold, double bb_, const NHParams& P) {
-    beta = rsold;
-    bb = bb_;
-    rtol = P.rtol;
-    rtol2bb = P.rtol * P.rtol * bb;
-    eps = P.eps;
-    max_it = P.max_it;
-    rr_prev = beta;
-    if (beta == 0.0) {  // :177
-      n = 0;
-      return kOk;
-    }
-    if (max_it < 1) {
-      n = 1;
-      status = PYOMGPU_MAXITER;
-      return kErr;
-    }
-    n = 1;
-    return kGo;
-  }
-  // after sweep A of iteration n: (s_n, A s_n) and max|s_n| over maskT
-  __device__ int after_a(double sAs, double smax, double& alpha) {
-    if (n > 1) {  // convergence test of iteration n-1 (:215-226)
-      const int m = n - 1;
-      const double step = fabs(alpha_prev) * smax;
-      if (m == 1) {
-        step1 = step;
-        est = step;
-        if (step < eps) {
-          n = m;
-          return kOk;
-        }
-      } else if (step < eps) {
-        const double rate = exp(log(step / step1) / (double)(m - 1));
-        est = step * rate / (1.0 - rate);
-        if (est < eps) {
-          n = m;
-          return kOk;
-        }
-      }
-      if (est != est) {
-        n = m;
-        status = PYOMGPU_NAN;
-        return kErr;
-      }
-      if (rtol > 0.0 && (bb > 0.0 ? rr_prev <= rtol2bb : rr_prev == 0.0)) {
-        est = sqrt(rr_prev);
-        n = m;
-        return kOk;
-      }
-      if (m >= max_it) {  // :228
-        n = max_it + 1;
-        status = PYOMGPU_MAXITER;
-        return kErr;
-      }
-    }
-    if (sAs == 0.0) return kOk;  // :185
-    alpha = beta / sAs;
-    return kGo;
-  }
-  // after sweep B of iteration n: rsnew = (res, res) over maskT
-  __device__ int after_b(double rsnew, double alpha) {
-    bq = rsnew / beta;  // p = res + rsnew/rsold*p (:189)
-    beta = rsnew;
-    if (n == 1) {  // divergence test (:197-205)
-      betamin = fabs(rsnew);
-    } else if (n > 2) {
-      betamin = fmin(betamin, fabs(rsnew));
-      if (fabs(rsnew) > 100.0 * betamin) {
-        status = PYOMGPU_DIVERGED;
-        return kErr;
-      }
-    }
-    alpha_prev = alpha;
-    rr_prev = rsnew;
-    ++n;
-    return kGo;
-  }
-  __device__ void finish(int how, CGResult* out) {
-    int converged = 0;
-    if (how == kOk) {
-      converged = 1;
-      status = PYOMGPU_OK;
-    } else if (est != est) {
-      status = PYOMGPU_NAN;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      out->iterations = n;
-      out->converged = converged;
-      out->status = status;
-      out->est = est;
-    }
-  }
-};
-
 template <bool CX, bool CY>
 __global__ void __launch_bounds__(kNHThreads, 2) nh_cg_kernel(const __grid_constant__ NHParams P) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -869,7 +764,9 @@ struct pyomgpu_nh {
   int grid = 0;        // 0: automatic
   int ty = 0, kc = 0;  // brick shape (0: automatic)
   int ns = 0;          // pipeline stages (0: automatic)
-  int variant = 0;     // 0 automatic, 1 brick kernel, 2 single-block kernel
+  int variant = 0;     // 0 automatic, 1 brick kernel, 2 cluster kernels
+  bool cut_planned = false;
+  pyomgpu::NHCut cut;  // cluster kernel (nh_clu.cu); npx = 0: the grid does not fit
   double timeout_s = 2.0;
   unsigned stall_next = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1161,6 +1058,68 @@ namespace {
 
 int nh_finish_cg(pyomgpu_nh* h, double* pdev, pyomgpu_solve_info* info, cudaStream_t st);
 
+void nh_clu_config(const NHCut& c, cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, cudaStream_t st) {
+  cfg.gridDim = dim3(c.npx * c.npy);
+  cfg.blockDim = dim3(c.nt);
+  cfg.dynamicSmemBytes = c.smem;
+  cfg.stream = st;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = c.npx * c.npy;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+}
+
+// Estimated iteration time (ns) of the cluster kernel on nb pieces of w x h
+// columns with nt threads of p levels.
+double nh_clu_iter_ns(int w, int h, int nz, int p, int nt, int nb) {
+  const double faces = nb == 1 ? 0.0 : 2.0 * (w + h) * nz / nt;  // records a thread sends and receives
+  if (nb == 1) return nt == 128 ? 900.0 + 90.0 * p : 1000.0 + 150.0 * p;
+  return 60.0 * faces + (nt == 128 ? 1050.0 + 130.0 * p + 20.0 * nb : 1100.0 + 180.0 * p + 42.0 * nb);
+}
+
+// Cut of the grid for the cluster kernel (nh_clu.cu), planned once: among the
+// cuts in x and y into at most kCluMaxBlocks pieces of whole columns that fit
+// its threads and shared memory, the one with the smallest estimated iteration
+// time.  False where none fits (about 49 000 cells at most) or the device
+// cannot place the cluster.
+bool nh_clu_plan(pyomgpu_nh* h) {
+  NHCut& best = h->cut;
+  if (h->cut_planned) return best.npx > 0;
+  h->cut_planned = true;
+  const int nx = h->G.g.nx, ny = h->G.g.ny, nz = h->G.nz;
+  const bool cx = h->cyclic_x != 0, cy = h->cyclic_y != 0;
+  double cost = 1e300;
+  for (int npx = 1; npx <= std::min(nx, kCluMaxBlocks); npx++)
+    for (int npy = 1; npy <= ny && npx * npy <= kCluMaxBlocks; npy++) {
+      const int w = (nx + npx - 1) / npx, hh = (ny + npy - 1) / npy;
+      for (const int* np : kNHCluNP) {
+        const int nt = np[0], p = np[1];
+        const size_t smem = nh_clu_smem_bytes(w, hh, nz, p);
+        if (smem > kNHSmallSmemMax || (size_t)w * hh * ((nz + p - 1) / p) > (size_t)nt) continue;
+        const double c = nh_clu_iter_ns(w, hh, nz, p, nt, npx * npy);
+        if (c < cost) {
+          cost = c;
+          best = NHCut{npx, npy, w, hh, p, nt, smem};
+        }
+      }
+    }
+  if (best.npx == 0) return false;
+  const void* k = nh_clu_kernel_ptr(best.nt, best.p, cx, cy);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  nh_clu_config(best, cfg, at, 0);
+  int n = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNHSmallSmemMax) != cudaSuccess ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    best = NHCut{};
+    return false;
+  }
+  return true;
+}
+
 // congrad_non_hydro on device arrays: fdev (forcing) and pdev (p_non_hydro(:,:,:,taup1), in/out), both
 // Fortran layout.  pdev may be a staging buffer whose result the caller copies out.
 int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int max_it, pyomgpu_solve_info* info,
@@ -1187,6 +1146,22 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
   h->stall_next = 0;
   P.out = h->d_result;
   const size_t ncell = (size_t)h->G.g.nx * h->G.g.ny * h->G.nz;
+  if (h->variant != 1 && nh_clu_plan(h)) {
+    const NHCut& c = h->cut;
+    P.cnpx = c.npx;
+    P.cnpy = c.npy;
+    P.cw = c.w;
+    P.ch = c.h;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    nh_clu_config(c, cfg, at, st);
+    void* cargs[] = {&P};
+    NCK(cudaEventRecord(h->e0, st));
+    NCK(cudaLaunchKernelExC(&cfg, nh_clu_kernel_ptr(c.nt, c.p, h->cyclic_x != 0, h->cyclic_y != 0), cargs));
+    NCK(cudaEventRecord(h->e1, st));
+    return nh_finish_cg(h, pdev, info, st);
+  }
+  // small grids the cluster kernel's threads or shared memory do not hold (deep or unusually shaped ones)
   const bool small = h->variant == 2 || (h->variant == 0 && ncell <= (size_t)kNHClusterAuto);
   if (small) {
     // cluster of C = 1, 2, 4, 8 or 16 blocks with about one cell per thread, each chunk within shared memory

@@ -21,6 +21,9 @@
 // products are summed in apply_op_3D's (kk, jj, ii) order with separately
 // rounded multiplies and adds, so A p is bit-identical to the reference's.
 #pragma once
+#include <math.h>
+
+#include "cg_clu.cuh"
 #include <cuda.h>
 #include <stdint.h>
 
@@ -149,7 +152,8 @@ struct alignas(64) NHParams {
   NHOp op;
   int ty, kw, kc;                    // brick shape
   int ns;                            // pipeline stages
-  int small_chunk;                   // cluster variant: cells per block
+  int small_chunk;                   // compact cluster kernel: cells per block
+  int cnpx, cnpy, cw, ch;            // cluster kernel: pieces in x and y, the largest piece
   int nbx, nby, nbz;                 // bricks per dimension
   const double* forc;  // Fortran layout (nx+4, ny+4, nz), device
   double* p;           // padded p_non_hydro(:,:,:,taup1), in/out
@@ -163,6 +167,116 @@ struct alignas(64) NHParams {
   unsigned long long timeout_ns;
   unsigned stall_extra;
   CGResult* out;
+};
+
+// Scalar state of congrad_non_hydro's loop (non_hydrostatic.f90:177-242),
+// the same in every thread of every block.  The convergence test of
+// iteration n needs max|p| of the direction formed after it, so it runs after
+// the next iteration's first sweep (after_a).
+struct NHCtl {
+  enum { kGo = 0, kOk = 1, kErr = 2 };
+  double beta = 0, bb = 0, rtol2bb = 0, eps = 0, rtol = 0;
+  double betamin = 0, step1 = 0, est = 0, bq = 0, alpha_prev = 0, rr_prev = 0;
+  int max_it = 0, n = 0, status = PYOMGPU_OK;
+
+  __device__ int start(double rsold, double bb_, const NHParams& P) {
+    beta = rsold;
+    bb = bb_;
+    rtol = P.rtol;
+    rtol2bb = P.rtol * P.rtol * bb;
+    eps = P.eps;
+    max_it = P.max_it;
+    rr_prev = beta;
+    if (beta == 0.0) {  // :177
+      n = 0;
+      return kOk;
+    }
+    if (max_it < 1) {
+      n = 1;
+      status = PYOMGPU_MAXITER;
+      return kErr;
+    }
+    n = 1;
+    return kGo;
+  }
+  // after sweep A of iteration n: (s_n, A s_n) and max|s_n| over maskT.  The quotient is formed beside the
+  // tests: it is what the next sweep waits for.
+  __device__ __forceinline__ int after_a(double sAs, double smax, double& alpha) {
+    const double quot = beta / sAs;
+    const double step = fabs(alpha_prev) * smax;
+    const int m = n - 1;
+    if ((m <= 1) | (step < eps) | (est != est) | (rtol > 0.0) | (m >= max_it) | (sAs == 0.0)) {
+      if (m >= 1) {  // convergence test of iteration n-1 (:215-226)
+        if (m == 1) {
+          step1 = step;
+          est = step;
+          if (step < eps) {
+            n = m;
+            return kOk;
+          }
+        } else if (step < eps) {
+          const double rate = exp(log(step / step1) / (double)(m - 1));
+          est = step * rate / (1.0 - rate);
+          if (est < eps) {
+            n = m;
+            return kOk;
+          }
+        }
+        if (est != est) {
+          n = m;
+          status = PYOMGPU_NAN;
+          return kErr;
+        }
+        if (rtol > 0.0 && (bb > 0.0 ? rr_prev <= rtol2bb : rr_prev == 0.0)) {
+          est = sqrt(rr_prev);
+          n = m;
+          return kOk;
+        }
+        if (m >= max_it) {  // :228
+          n = max_it + 1;
+          status = PYOMGPU_MAXITER;
+          return kErr;
+        }
+      }
+      if (sAs == 0.0) return kOk;  // :185
+    }
+    alpha = quot;
+    return kGo;
+  }
+  // after sweep B of iteration n: rsnew = (res, res) over maskT
+  __device__ __forceinline__ int after_b(double rsnew, double alpha) {
+    bq = rsnew / beta;  // p = res + rsnew/rsold*p (:189)
+    beta = rsnew;
+    const double low = fmin(betamin, fabs(rsnew));
+    if (n == 1) {  // divergence test (:197-205)
+      betamin = fabs(rsnew);
+    } else if (n > 2) {
+      betamin = low;
+      if (fabs(rsnew) > 100.0 * low) {
+        status = PYOMGPU_DIVERGED;
+        return kErr;
+      }
+    }
+    alpha_prev = alpha;
+    rr_prev = rsnew;
+    ++n;
+    return kGo;
+  }
+  __device__ void finish(int how, CGResult* out) {
+    int converged = 0;
+    if (how == kOk) {
+      converged = 1;
+      status = PYOMGPU_OK;
+    } else if (est != est) {
+      status = PYOMGPU_NAN;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      out->iterations = n;
+      out->converged = converged;
+      out->status = status;
+      out->est = est;
+    }
+  }
 };
 
 // Arrays of one solve_non_hydrostatic step (non_hydrostatic.f90:5-63), all
@@ -195,6 +309,19 @@ constexpr int kNHSmallMaxChunk = (int)(kNHSmallSmemMax / 33);
 constexpr int kNHSmallMaxCells = kNHMaxCluster * kNHSmallMaxChunk;
 constexpr int kNHClusterAuto = 32768;  // automatic choice: the cluster kernel up to this many cells
 const void* nh_cg_small_kernel_ptr(bool cyclic_x, bool cyclic_y);
+
+// cluster kernel (nh_clu.cu): pieces of whole columns in the registers and shared memory of one cluster
+struct NHCut {
+  int npx = 0, npy = 0, w = 0, h = 0, p = 0, nt = 0;
+  size_t smem = 0;
+};
+constexpr int kNHCluNP[][2] = {{128, 4}, {128, 8}, {256, 4}, {256, 8}, {256, 12}};  // threads, levels per thread
+// direction with its rim, vertical factors, staged faces, received records (4 words each), reduction slots
+__host__ __device__ constexpr size_t nh_clu_smem_bytes(int w, int h, int nz, int p) {
+  return 8 * ((size_t)(w + 2) * (h + 2) * ((nz + p - 1) / p * p + 2) + 2 * (size_t)((nz + p - 1) / p * p) +
+              4 * (size_t)(w + h) * nz) + 16 + 64 * (size_t)(w + h) * nz + 8 * (size_t)kCluMaxSlots * 16;
+}
+const void* nh_clu_kernel_ptr(int nt, int p, bool cyclic_x, bool cyclic_y);
 void launch_nh_apply(const NHGeo& G, const NHOp& op, const double* p, double* res, cudaStream_t st);
 void launch_nh_pack(const NHGeo& G, const double* user, double* padded, cudaStream_t st);
 void launch_nh_unpack(const NHGeo& G, const double* padded, double* user, cudaStream_t st);
