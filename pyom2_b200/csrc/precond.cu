@@ -56,6 +56,7 @@ struct pyomgpu_precond {
   double *r = nullptr, *w1 = nullptr, *w2 = nullptr, *aw1 = nullptr, *aw2 = nullptr;
   double *p1 = nullptr, *p2 = nullptr, *ap1 = nullptr, *ap2 = nullptr, *t1 = nullptr, *t2 = nullptr;
   double* part = nullptr;  // per-block partials
+  unsigned* arrived = nullptr;  // blocks that have left their partials (grid_totals)
   double* sc = nullptr;    // device scalars
   double* h_sc = nullptr;  // pinned copy
   float* gz = nullptr;     // [Hp][Wp]
@@ -90,16 +91,19 @@ __device__ __forceinline__ double dweight(const double* dxu, const double* dyu, 
   return dxu[i + 1] * dyu[j + 1] * cosu[j + 1];
 }
 
-// Block partial sums of NV values, written to part[blockIdx.x * NV + k].
+// Sums of NV values over the grid (fixed order), given to thread 0 of the block
+// that finishes last: every block leaves its partial sums in part, and the last
+// to count itself in at `arrived` adds them up and clears the counter.  True in
+// every thread of that block.  (A launch of one warp for it took 6 us, three of
+// them an iteration: the partials one load after another.)
 template <int NV>
-__device__ __forceinline__ void block_partials(double (&v)[NV], double* part) {
+__device__ __forceinline__ bool grid_totals(const double (&v)[NV], double* part, unsigned* arrived, double (&out)[NV]) {
   __shared__ double sh[kRB / 32][NV];
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < NV; k++) {
-    double x = v[k];
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+    const double x = warp_sum(v[k]);
     if (lane == 0) sh[w][k] = x;
   }
   __syncthreads();
@@ -107,192 +111,36 @@ __device__ __forceinline__ void block_partials(double (&v)[NV], double* part) {
     double s = 0.0;
     for (int q = 0; q < kRB / 32; q++) s += sh[q][threadIdx.x];
     part[blockIdx.x * NV + threadIdx.x] = s;
+    __threadfence();
   }
-}
-
-// Sum of the partials of nv values (fixed order) into out[0..nv), by one warp.
-__device__ __forceinline__ void sum_partials(const double* __restrict__ part, int nb, int nv, double* out) {
-  double v[kMaxNV] = {0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nb; b += 32)
-    for (int k = 0; k < nv; k++) v[k] += part[b * nv + k];
-  for (int k = 0; k < nv; k++) {
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(arrived, 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double t[NV];
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], m);
-    out[k] = v[k];
+  for (int k = 0; k < NV; k++) t[k] = 0.0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += kRB)
+#pragma unroll
+    for (int k = 0; k < NV; k++) t[k] += __ldcg(part + (size_t)b * NV + k);
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const double x = warp_sum(t[k]);
+    if (lane == 0) sh[w][k] = x;
   }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    out[k] = 0.0;
+    for (int q = 0; q < kRB / 32; q++) out[k] += sh[q][k];
+  }
+  if (threadIdx.x == 0) *arrived = 0u;
+  return true;
 }
 
 __global__ void k_set_scalar(double* sc, int idx, double v) {
   if (threadIdx.x == 0 && blockIdx.x == 0) sc[idx] = v;
-}
-
-// ---------------------------------------------------------------- image <-> field
-__global__ void k_static(Geo g, const double* __restrict__ W, const double* __restrict__ hur,
-                         const double* __restrict__ cosu, double hur_scale, int Hp, int Wp, float4* __restrict__ stat) {
-  const size_t n = (size_t)Hp * Wp;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int y = (int)(e / Wp), x = (int)(e - (size_t)y * Wp);
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (x < g.nx && y < g.ny) {
-      const int i = x + 1, j = y + 1;
-      const bool m = W[g.at(i, j)] != 0.0;
-      s.x = m ? 1.f : 0.f;
-      s.y = m ? (float)(hur[fidx(g.nx, i, j)] * hur_scale) : 0.f;
-      s.z = (float)cosu[j + 1];
-    }
-    stat[e] = s;
-  }
-}
-
-__device__ __forceinline__ uint16_t f2bf_rn(float f) {
-  uint32_t u = __float_as_uint(f);
-  u += 0x7FFFu + ((u >> 16) & 1u);
-  return (uint16_t)(u >> 16);
-}
-
-// X0 group 0 = (r / rms(r) masked, mask, hur, cos, 0, 0, 0, 0)
-__global__ void k_prep(Geo g, const double* __restrict__ r, const double* __restrict__ sc, double nu,
-                       const float4* __restrict__ stat, int Hp, int Wp, uint16_t* __restrict__ X0) {
-  if (sc[kDone] != 0.0) return;
-  const double rr = sc[kRR];
-  const double inv = rr > 0.0 ? 1.0 / sqrt(rr / nu) : 0.0;
-  const size_t n = (size_t)Hp * Wp;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int y = (int)(e / Wp), x = (int)(e - (size_t)y * Wp);
-    const float4 s = stat[e];
-    float rv = 0.f;
-    if (x < g.nx && y < g.ny && s.x != 0.f) rv = (float)(r[g.at(x + 1, y + 1)] * inv);
-    uint4 o;
-    o.x = (uint32_t)f2bf_rn(rv) | ((uint32_t)f2bf_rn(s.x) << 16);
-    o.y = (uint32_t)f2bf_rn(s.y) | ((uint32_t)f2bf_rn(s.z) << 16);
-    o.z = 0u;
-    o.w = 0u;
-    reinterpret_cast<uint4*>(X0)[e] = o;
-  }
-}
-
-// w1 = Z r (Jacobi direction), w2 = mask * network output (cyclic copies)
-__global__ void k_dirs(Geo g, const float* __restrict__ zn, const float4* __restrict__ stat, int Wp,
-                       const double* __restrict__ Z, const double* __restrict__ r, const double* __restrict__ sc,
-                       double* __restrict__ w1, double* __restrict__ w2) {
-  if (sc[kDone] != 0.0) return;
-  const size_t n = (size_t)g.nx * g.ny;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int y = (int)(e / g.nx), x = (int)(e - (size_t)y * g.nx);
-    const size_t pi = (size_t)y * Wp + x, k = g.at(x + 1, y + 1);
-    store_cyclic(w1, g, x + 1, y + 1, Z[k] * r[k]);
-    store_cyclic(w2, g, x + 1, y + 1, stat[pi].x != 0.f ? (double)zn[pi] : 0.0);
-  }
-}
-
-// aw = A w for both directions; partials <A p_i, w_j>_D (previous block)
-__global__ void k_apply_w(Geo g, OpDev<double> op, const double* __restrict__ w1, const double* __restrict__ w2,
-                          const double* __restrict__ ap1, const double* __restrict__ ap2, const double* dxu,
-                          const double* dyu, const double* cosu, const double* __restrict__ sc,
-                          double* __restrict__ aw1, double* __restrict__ aw2, double* __restrict__ part) {
-  double v[4] = {0, 0, 0, 0};
-  if (sc[kDone] == 0.0) {
-    const size_t n = (size_t)g.nx * g.ny;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-      const int j = (int)(e / g.nx) + 1, i = (int)(e - (size_t)(j - 1) * g.nx) + 1;
-      const size_t k = g.at(i, j);
-      aw1[k] = apply_point(op, g, w1, i, j);
-      aw2[k] = apply_point(op, g, w2, i, j);
-      const double d = dweight(dxu, dyu, cosu, i, j);
-      const double a1 = d * ap1[k], a2 = d * ap2[k];
-      v[0] += a1 * w1[k];
-      v[1] += a1 * w2[k];
-      v[2] += a2 * w1[k];
-      v[3] += a2 * w2[k];
-    }
-  }
-  block_partials<4>(v, part);
-}
-
-// P_new = W - P B, AP_new = AW - AP B (in place); partials <p1,ap1>, <p1,ap2>, <p2,ap2>, <p1,r>, <p2,r> (D)
-__global__ void k_new_block(Geo g, const double* __restrict__ w1, const double* __restrict__ w2,
-                            const double* __restrict__ aw1, const double* __restrict__ aw2,
-                            const double* __restrict__ r, const double* dxu, const double* dyu, const double* cosu,
-                            const double* __restrict__ sc, double* __restrict__ p1, double* __restrict__ p2,
-                            double* __restrict__ ap1, double* __restrict__ ap2, double* __restrict__ part) {
-  double v[5] = {0, 0, 0, 0, 0};
-  if (sc[kDone] == 0.0) {
-    const double b11 = sc[kB11], b12 = sc[kB12], b21 = sc[kB21], b22 = sc[kB22];
-    const size_t n = (size_t)g.nx * g.ny;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-      const int j = (int)(e / g.nx) + 1, i = (int)(e - (size_t)(j - 1) * g.nx) + 1;
-      const size_t k = g.at(i, j);
-      const double po1 = p1[k], po2 = p2[k], qo1 = ap1[k], qo2 = ap2[k];
-      const double n1 = w1[k] - (po1 * b11 + po2 * b21), n2 = w2[k] - (po1 * b12 + po2 * b22);
-      const double m1 = aw1[k] - (qo1 * b11 + qo2 * b21), m2 = aw2[k] - (qo1 * b12 + qo2 * b22);
-      store_cyclic(p1, g, i, j, n1);
-      store_cyclic(p2, g, i, j, n2);
-      ap1[k] = m1;
-      ap2[k] = m2;
-      const double d = dweight(dxu, dyu, cosu, i, j);
-      v[0] += d * n1 * m1;
-      v[1] += d * n1 * m2;
-      v[2] += d * n2 * m2;
-      v[3] += d * n1 * r[k];
-      v[4] += d * n2 * r[k];
-    }
-  }
-  block_partials<5>(v, part);
-}
-
-// x += c1 p1 + c2 p2, r -= c1 ap1 + c2 ap2 (unknowns); partial sum r^2
-__global__ void k_step(Geo g, const double* __restrict__ W, const double* __restrict__ p1,
-                       const double* __restrict__ p2, const double* __restrict__ ap1, const double* __restrict__ ap2,
-                       const double* __restrict__ sc, double* __restrict__ x, double* __restrict__ r,
-                       double* __restrict__ part) {
-  double v[1] = {0.0};
-  if (sc[kDone] == 0.0) {
-    const double c1 = sc[kC1], c2 = sc[kC2];
-    const size_t n = (size_t)g.nx * g.ny;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-      const int j = (int)(e / g.nx) + 1, i = (int)(e - (size_t)(j - 1) * g.nx) + 1;
-      const size_t k = g.at(i, j);
-      if (W[k] == 0.0) continue;
-      x[k] += c1 * p1[k] + c2 * p2[k];
-      const double rv = r[k] - (c1 * ap1[k] + c2 * ap2[k]);
-      store_cyclic(r, g, i, j, rv);
-      v[0] += rv * rv;
-    }
-  }
-  block_partials<1>(v, part);
-}
-
-// r = mask (forc - A x); partials sum r^2, sum forc^2 over the unknowns
-__global__ void k_residual_vec(Geo g, OpDev<double> op, const double* __restrict__ forc, const double* __restrict__ x,
-                               double* __restrict__ r, double* __restrict__ part) {
-  double v[2] = {0.0, 0.0};
-  const size_t n = (size_t)g.nx * g.ny;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e / g.nx) + 1, i = (int)(e - (size_t)(j - 1) * g.nx) + 1;
-    const bool m = op.W[g.at(i, j)] != 0.0;
-    const double f = forc[fidx(g.nx, i, j)];
-    const double rv = m ? f - apply_point(op, g, x, i, j) : 0.0;
-    store_cyclic(r, g, i, j, rv);
-    if (m) {
-      v[0] += rv * rv;
-      v[1] += f * f;
-    }
-  }
-  block_partials<2>(v, part);
-}
-
-// r_pad = mask * r_user (cyclic copies); partial sum r^2 over the unknowns
-__global__ void k_mask_rr(Geo g, const double* __restrict__ W, const double* __restrict__ r_user,
-                          double* __restrict__ r, double* __restrict__ part) {
-  double v[1] = {0.0};
-  const size_t n = (size_t)g.nx * g.ny;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e / g.nx) + 1, i = (int)(e - (size_t)(j - 1) * g.nx) + 1;
-    const double rv = W[g.at(i, j)] != 0.0 ? r_user[fidx(g.nx, i, j)] : 0.0;
-    store_cyclic(r, g, i, j, rv);
-    v[0] += rv * rv;
-  }
-  block_partials<1>(v, part);
 }
 
 // 2x2 symmetric solve G c = h; rank 1 (second direction dropped) when G is
@@ -313,12 +161,9 @@ __device__ int solve2(double g11, double g12, double g22, double h1, double h2, 
   return 0;
 }
 
-// stage 0: initial residual; 1: T -> B; 2: G, h -> c; 3: rr -> done?; 4: rr only
-__global__ void k_scalars(const double* __restrict__ part, int nb, int stage, double* __restrict__ sc) {
-  const int nv = stage == 0 ? 2 : stage == 1 ? 4 : stage == 2 ? 5 : 1;
-  double s[kMaxNV];
-  sum_partials(part, nb, nv, s);
-  if (threadIdx.x != 0) return;
+// Scalar step on the totals s, by one thread.  stage 0: initial residual; 1: T -> B; 2: G, h -> c;
+// 3: rr -> done?; 4: rr only
+__device__ void scalar_step(const double* s, int stage, double* __restrict__ sc) {
   if (stage == 0) {
     sc[kRR] = s[0];
     sc[kBB] = s[1];
@@ -385,6 +230,207 @@ __global__ void k_scalars(const double* __restrict__ part, int nb, int stage, do
   }
 }
 
+// ---------------------------------------------------------------- image <-> field
+__global__ void k_static(Geo g, const double* __restrict__ W, const double* __restrict__ hur,
+                         const double* __restrict__ cosu, double hur_scale, int Hp, int Wp, float4* __restrict__ stat) {
+  const size_t n = (size_t)Hp * Wp;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const int y = (int)(e / Wp), x = (int)(e - (size_t)y * Wp);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (x < g.nx && y < g.ny) {
+      const int i = x + 1, j = y + 1;
+      const bool m = W[g.at(i, j)] != 0.0;
+      s.x = m ? 1.f : 0.f;
+      s.y = m ? (float)(hur[fidx(g.nx, i, j)] * hur_scale) : 0.f;
+      s.z = (float)cosu[j + 1];
+    }
+    stat[e] = s;
+  }
+}
+
+__device__ __forceinline__ uint16_t f2bf_rn(float f) {
+  uint32_t u = __float_as_uint(f);
+  u += 0x7FFFu + ((u >> 16) & 1u);
+  return (uint16_t)(u >> 16);
+}
+
+// X0 group 0 = (r / rms(r) masked, mask, hur, cos, 0, 0, 0, 0)
+__global__ void k_prep(Geo g, const double* __restrict__ r, const double* __restrict__ sc, double nu,
+                       const float4* __restrict__ stat, int Hp, int Wp, uint16_t* __restrict__ X0) {
+  if (sc[kDone] != 0.0) return;
+  const double rr = sc[kRR];
+  const double inv = rr > 0.0 ? 1.0 / sqrt(rr / nu) : 0.0;
+  const size_t n = (size_t)Hp * Wp;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const int y = (int)(e / Wp), x = (int)(e - (size_t)y * Wp);
+    const float4 s = stat[e];
+    float rv = 0.f;
+    if (x < g.nx && y < g.ny && s.x != 0.f) rv = (float)(r[g.at(x + 1, y + 1)] * inv);
+    uint4 o;
+    o.x = (uint32_t)f2bf_rn(rv) | ((uint32_t)f2bf_rn(s.x) << 16);
+    o.y = (uint32_t)f2bf_rn(s.y) | ((uint32_t)f2bf_rn(s.z) << 16);
+    o.z = 0u;
+    o.w = 0u;
+    reinterpret_cast<uint4*>(X0)[e] = o;
+  }
+}
+
+// w1 = Z r (Jacobi direction), w2 = mask * network output (cyclic copies)
+__global__ void k_dirs(Geo g, const float* __restrict__ zn, const float4* __restrict__ stat, int Wp,
+                       const double* __restrict__ Z, const double* __restrict__ r, const double* __restrict__ sc,
+                       double* __restrict__ w1, double* __restrict__ w2) {
+  if (sc[kDone] != 0.0) return;
+  const size_t n = (size_t)g.nx * g.ny;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const int y = (int)(e / g.nx), x = (int)(e - (size_t)y * g.nx);
+    const size_t pi = (size_t)y * Wp + x, k = g.at(x + 1, y + 1);
+    store_cyclic(w1, g, x + 1, y + 1, Z[k] * r[k]);
+    store_cyclic(w2, g, x + 1, y + 1, stat[pi].x != 0.f ? (double)zn[pi] : 0.0);
+  }
+}
+
+// The two new directions at (i, j), formed where they are read: w1 = Z r
+// (Jacobi; Z and r have valid cyclic halos) and w2 = mask * network output
+// (image of the interior, wrapped like setcyclic_xy; no points beyond a closed
+// side).  Z is 0 exactly where the mask is.
+struct Dirs {
+  const double *Z, *r;
+  const float* zn;
+  int Wp;
+  __device__ __forceinline__ double w1(const Geo& g, int i, int j) const { return Z[g.at(i, j)] * r[g.at(i, j)]; }
+  __device__ __forceinline__ double w2(const Geo& g, int i, int j) const {
+    if (Z[g.at(i, j)] == 0.0) return 0.0;
+    if (i < 1 || i > g.nx) {
+      if (!g.cyclic_x) return 0.0;
+      i += i < 1 ? g.nx : -g.nx;
+    }
+    if (j < 1 || j > g.ny) {
+      if (!g.cyclic_y) return 0.0;
+      j += j < 1 ? g.ny : -g.ny;
+    }
+    return (double)zn[(size_t)(j - 1) * Wp + (i - 1)];
+  }
+};
+
+// aw = A w for both directions; partials <A p_i, w_j>_D (previous block)
+__global__ void k_apply_w(Geo g, OpDev<double> op, Dirs d, const double* __restrict__ ap1,
+                          const double* __restrict__ ap2, const double* dxu, const double* dyu, const double* cosu,
+                          double* sc, double* __restrict__ aw1, double* __restrict__ aw2, double* __restrict__ part,
+                          unsigned* __restrict__ arrived) {
+  double v[4] = {0, 0, 0, 0};
+  if (sc[kDone] == 0.0) {
+    const unsigned n = (unsigned)g.nx * g.ny;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+      const int j = (int)(e / (unsigned)g.nx) + 1, i = (int)(e - (unsigned)(j - 1) * g.nx) + 1;
+      const size_t k = g.at(i, j);
+      const double sx = op.ax[i + 1] * op.bx[j + 1], sy = op.by[j + 1];
+      const double fe = op.FX[g.at(i + 1, j)], fw = op.FX[k], fn = op.FY[g.at(i, j + 1)], fs = op.FY[k];
+      const double c1 = d.w1(g, i, j), c2 = d.w2(g, i, j);
+      aw1[k] = sx * (fe * (d.w1(g, i + 1, j) - c1) + fw * (d.w1(g, i - 1, j) - c1)) +
+               sy * (fn * (d.w1(g, i, j + 1) - c1) + fs * (d.w1(g, i, j - 1) - c1));
+      aw2[k] = sx * (fe * (d.w2(g, i + 1, j) - c2) + fw * (d.w2(g, i - 1, j) - c2)) +
+               sy * (fn * (d.w2(g, i, j + 1) - c2) + fs * (d.w2(g, i, j - 1) - c2));
+      const double D = dweight(dxu, dyu, cosu, i, j);
+      const double a1 = D * ap1[k], a2 = D * ap2[k];
+      v[0] += a1 * c1;
+      v[1] += a1 * c2;
+      v[2] += a2 * c1;
+      v[3] += a2 * c2;
+    }
+  }
+  double tot[4];
+  if (grid_totals<4>(v, part, arrived, tot) && threadIdx.x == 0) scalar_step(tot, 1, sc);
+}
+
+// P_new = W - P B, AP_new = AW - AP B (in place); partials <p1,ap1>, <p1,ap2>, <p2,ap2>, <p1,r>, <p2,r> (D)
+__global__ void k_new_block(Geo g, Dirs dd, const double* __restrict__ aw1, const double* __restrict__ aw2,
+                            const double* __restrict__ r, const double* dxu, const double* dyu, const double* cosu,
+                            double* sc, double* __restrict__ p1, double* __restrict__ p2,
+                            double* __restrict__ ap1, double* __restrict__ ap2, double* __restrict__ part, unsigned* __restrict__ arrived) {
+  double v[5] = {0, 0, 0, 0, 0};
+  if (sc[kDone] == 0.0) {
+    const double b11 = sc[kB11], b12 = sc[kB12], b21 = sc[kB21], b22 = sc[kB22];
+    const unsigned n = (unsigned)g.nx * g.ny;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+      const int j = (int)(e / (unsigned)g.nx) + 1, i = (int)(e - (unsigned)(j - 1) * g.nx) + 1;
+      const size_t k = g.at(i, j);
+      const double po1 = p1[k], po2 = p2[k], qo1 = ap1[k], qo2 = ap2[k];
+      const double n1 = dd.w1(g, i, j) - (po1 * b11 + po2 * b21), n2 = dd.w2(g, i, j) - (po1 * b12 + po2 * b22);
+      const double m1 = aw1[k] - (qo1 * b11 + qo2 * b21), m2 = aw2[k] - (qo1 * b12 + qo2 * b22);
+      store_cyclic(p1, g, i, j, n1);
+      store_cyclic(p2, g, i, j, n2);
+      ap1[k] = m1;
+      ap2[k] = m2;
+      const double d = dweight(dxu, dyu, cosu, i, j);
+      v[0] += d * n1 * m1;
+      v[1] += d * n1 * m2;
+      v[2] += d * n2 * m2;
+      v[3] += d * n1 * r[k];
+      v[4] += d * n2 * r[k];
+    }
+  }
+  double tot[5];
+  if (grid_totals<5>(v, part, arrived, tot) && threadIdx.x == 0) scalar_step(tot, 2, sc);
+}
+
+// x += c1 p1 + c2 p2, r -= c1 ap1 + c2 ap2 (unknowns); partial sum r^2
+__global__ void k_step(Geo g, const double* __restrict__ W, const double* __restrict__ p1,
+                       const double* __restrict__ p2, const double* __restrict__ ap1, const double* __restrict__ ap2,
+                       double* sc, double* __restrict__ x, double* __restrict__ r,
+                       double* __restrict__ part, unsigned* __restrict__ arrived) {
+  double v[1] = {0.0};
+  if (sc[kDone] == 0.0) {
+    const double c1 = sc[kC1], c2 = sc[kC2];
+    const unsigned n = (unsigned)g.nx * g.ny;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+      const int j = (int)(e / (unsigned)g.nx) + 1, i = (int)(e - (unsigned)(j - 1) * g.nx) + 1;
+      const size_t k = g.at(i, j);
+      if (W[k] == 0.0) continue;
+      x[k] += c1 * p1[k] + c2 * p2[k];
+      const double rv = r[k] - (c1 * ap1[k] + c2 * ap2[k]);
+      store_cyclic(r, g, i, j, rv);
+      v[0] += rv * rv;
+    }
+  }
+  double tot[1];
+  if (grid_totals<1>(v, part, arrived, tot) && threadIdx.x == 0) scalar_step(tot, 3, sc);
+}
+
+// r = mask (forc - A x); partials sum r^2, sum forc^2 over the unknowns
+__global__ void k_residual_vec(Geo g, OpDev<double> op, const double* __restrict__ forc, const double* __restrict__ x,
+                               double* __restrict__ r, double* __restrict__ part, unsigned* __restrict__ arrived, double* __restrict__ sc) {
+  double v[2] = {0.0, 0.0};
+  const unsigned n = (unsigned)g.nx * g.ny;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int j = (int)(e / (unsigned)g.nx) + 1, i = (int)(e - (unsigned)(j - 1) * g.nx) + 1;
+    const bool m = op.W[g.at(i, j)] != 0.0;
+    const double f = forc[fidx(g.nx, i, j)];
+    const double rv = m ? f - apply_point(op, g, x, i, j) : 0.0;
+    store_cyclic(r, g, i, j, rv);
+    if (m) {
+      v[0] += rv * rv;
+      v[1] += f * f;
+    }
+  }
+  double tot[2];
+  if (grid_totals<2>(v, part, arrived, tot) && threadIdx.x == 0) scalar_step(tot, 0, sc);
+}
+
+// r_pad = mask * r_user (cyclic copies); partial sum r^2 over the unknowns
+__global__ void k_mask_rr(Geo g, const double* __restrict__ W, const double* __restrict__ r_user,
+                          double* __restrict__ r, double* __restrict__ part, unsigned* __restrict__ arrived, double* __restrict__ sc) {
+  double v[1] = {0.0};
+  const unsigned n = (unsigned)g.nx * g.ny;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int j = (int)(e / (unsigned)g.nx) + 1, i = (int)(e - (unsigned)(j - 1) * g.nx) + 1;
+    const double rv = W[g.at(i, j)] != 0.0 ? r_user[fidx(g.nx, i, j)] : 0.0;
+    store_cyclic(r, g, i, j, rv);
+    v[0] += rv * rv;
+  }
+  double tot[1];
+  if (grid_totals<1>(v, part, arrived, tot) && threadIdx.x == 0) scalar_step(tot, 4, sc);
+}
+
 // ---------------------------------------------------------------- training loss
 // Zp = mask * zn, Ep = mask * e * scale (padded FP64 with cyclic copies), scale = dbar / rms(r)
 __global__ void k_loss_fields(Geo g, const float* __restrict__ zn, const double* __restrict__ e_user,
@@ -401,14 +447,23 @@ __global__ void k_loss_fields(Geo g, const float* __restrict__ zn, const double*
   }
 }
 
+// loss = (b - 2a + c) / c (all three are S forms, S negative definite); d loss / d z = (2/c)(S z - S e)
+__device__ void loss_scalars(const double* s, double* __restrict__ sc) {
+  const double a = s[0], b = s[1], c = s[2];
+  const bool ok = c != 0.0 && a == a && b == b && c == c;
+  sc[kLoss] = ok ? (b - 2.0 * a + c) / c : 1.0;
+  sc[kK1] = ok ? 2.0 / c : 0.0;
+  sc[kK2] = ok ? -2.0 / c : 0.0;
+}
+
 // SZ = D A Zp, SE = D A Ep; partials a = z^T S e, b = z^T S z, c = e^T S e
 __global__ void k_loss_dots(Geo g, OpDev<double> op, const double* __restrict__ Zp, const double* __restrict__ Ep,
                             const double* dxu, const double* dyu, const double* cosu, double* __restrict__ SZ,
-                            double* __restrict__ SE, double* __restrict__ part) {
+                            double* __restrict__ SE, double* __restrict__ part, unsigned* __restrict__ arrived, double* __restrict__ sc) {
   double v[3] = {0.0, 0.0, 0.0};
-  const size_t n = (size_t)g.nx * g.ny;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int j = (int)(e / g.nx) + 1, i = (int)(e - (size_t)(j - 1) * g.nx) + 1;
+  const unsigned n = (unsigned)g.nx * g.ny;
+  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int j = (int)(e / (unsigned)g.nx) + 1, i = (int)(e - (unsigned)(j - 1) * g.nx) + 1;
     const size_t k = g.at(i, j);
     const double d = dweight(dxu, dyu, cosu, i, j);
     const double sz = d * apply_point(op, g, Zp, i, j), se = d * apply_point(op, g, Ep, i, j);
@@ -418,19 +473,8 @@ __global__ void k_loss_dots(Geo g, OpDev<double> op, const double* __restrict__ 
     v[1] += Zp[k] * sz;
     v[2] += Ep[k] * se;
   }
-  block_partials<3>(v, part);
-}
-
-// loss = (b - 2a + c) / c (all three are S forms, S negative definite); d loss / d z = (2/c)(S z - S e)
-__global__ void k_loss_scalars(const double* __restrict__ part, int nb, double* __restrict__ sc) {
-  double s[kMaxNV];
-  sum_partials(part, nb, 3, s);
-  if (threadIdx.x != 0) return;
-  const double a = s[0], b = s[1], c = s[2];
-  const bool ok = c != 0.0 && a == a && b == b && c == c;
-  sc[kLoss] = ok ? (b - 2.0 * a + c) / c : 1.0;
-  sc[kK1] = ok ? 2.0 / c : 0.0;
-  sc[kK2] = ok ? -2.0 / c : 0.0;
+  double tot[3];
+  if (grid_totals<3>(v, part, arrived, tot) && threadIdx.x == 0) loss_scalars(tot, sc);
 }
 
 __global__ void k_loss_grad(Geo g, const double* __restrict__ SZ, const double* __restrict__ SE,
@@ -472,8 +516,7 @@ bool is_dev(const void* p) {
 void load_r(pyomgpu_precond* P, const double* r_user, cudaStream_t st) {
   const Geo& g = P->c->g;
   const int nb = blocks_for((size_t)g.nx * g.ny);
-  k_mask_rr<<<nb, kRB, 0, st>>>(g, P->c->sf.W, r_user, P->r, P->part);
-  k_scalars<<<1, 32, 0, st>>>(P->part, nb, 4, P->sc);
+  k_mask_rr<<<nb, kRB, 0, st>>>(g, P->c->sf.W, r_user, P->r, P->part, P->arrived, P->sc);
   k_set_scalar<<<1, 1, 0, st>>>(P->sc, kDone, 0.0);
 }
 
@@ -490,18 +533,15 @@ int iteration(pyomgpu_precond* P, cudaStream_t st) {
   const Geo& g = c->g;
   const int nb = blocks_for((size_t)g.nx * g.ny);
   if (int rc = run_net(P, st)) return rc;
-  k_dirs<<<nb, kRB, 0, st>>>(g, P->net.z, P->stat, P->Wp, c->sf.W, P->r, P->sc, P->w1, P->w2);
-  k_apply_w<<<nb, kRB, 0, st>>>(g, c->sf.dev(), P->w1, P->w2, P->ap1, P->ap2, c->dxu, c->dyu, c->cosu, P->sc, P->aw1,
-                                P->aw2, P->part);
-  k_scalars<<<1, 32, 0, st>>>(P->part, nb, 1, P->sc);
-  k_new_block<<<nb, kRB, 0, st>>>(g, P->w1, P->w2, P->aw1, P->aw2, P->r, c->dxu, c->dyu, c->cosu, P->sc, P->p1,
-                                  P->p2, P->ap1, P->ap2, P->part);
-  k_scalars<<<1, 32, 0, st>>>(P->part, nb, 2, P->sc);
-  k_step<<<nb, kRB, 0, st>>>(g, c->sf.W, P->p1, P->p2, P->ap1, P->ap2, P->sc, c->sol, P->r, P->part);
-  k_scalars<<<1, 32, 0, st>>>(P->part, nb, 3, P->sc);
+  const Dirs d{c->sf.W, P->r, P->net.z, P->Wp};
+  k_apply_w<<<nb, kRB, 0, st>>>(g, c->sf.dev(), d, P->ap1, P->ap2, c->dxu, c->dyu, c->cosu, P->sc, P->aw1, P->aw2,
+                                P->part, P->arrived);
+  k_new_block<<<nb, kRB, 0, st>>>(g, d, P->aw1, P->aw2, P->r, c->dxu, c->dyu, c->cosu, P->sc, P->p1, P->p2, P->ap1,
+                                  P->ap2, P->part, P->arrived);
+  k_step<<<nb, kRB, 0, st>>>(g, c->sf.W, P->p1, P->p2, P->ap1, P->ap2, P->sc, c->sol, P->r, P->part, P->arrived);
   return (int)cudaGetLastError();
 }
-constexpr int kLaunchesPerIteration = 1 + kUNetLayers + 7;
+constexpr int kLaunchesPerIteration = 1 + kUNetLayers + 3;
 
 int ensure_graph(pyomgpu_precond* P) {
   if (P->exec) return 0;
@@ -578,6 +618,8 @@ int32_t pyomgpu_precond_create(pyomgpu_ctx* c, int32_t training, pyomgpu_precond
          cudaMemset(*a, 0, Pn * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc((void**)&P->stat, npx * sizeof(float4)) == cudaSuccess &&
        cudaMalloc((void**)&P->part, (size_t)kRBlocks * kMaxNV * sizeof(double)) == cudaSuccess &&
+       cudaMalloc((void**)&P->arrived, sizeof(unsigned)) == cudaSuccess &&
+       cudaMemset(P->arrived, 0, sizeof(unsigned)) == cudaSuccess &&
        cudaMalloc((void**)&P->sc, kNSc * sizeof(double)) == cudaSuccess &&
        cudaMallocHost((void**)&P->h_sc, kNSc * sizeof(double)) == cudaSuccess &&
        cudaMalloc((void**)&P->gz, npx * sizeof(float)) == cudaSuccess;
@@ -614,7 +656,7 @@ void pyomgpu_precond_destroy(pyomgpu_precond* P) {
   unet_free(P->net);
   for (void* a : {(void*)P->r, (void*)P->w1, (void*)P->w2, (void*)P->aw1, (void*)P->aw2, (void*)P->p1, (void*)P->p2,
                   (void*)P->ap1, (void*)P->ap2, (void*)P->t1, (void*)P->t2, (void*)P->stat, (void*)P->part,
-                  (void*)P->sc, (void*)P->gz})
+                  (void*)P->sc, (void*)P->gz, (void*)P->arrived})
     if (a) cudaFree(a);
   if (P->h_sc) cudaFreeHost(P->h_sc);
   delete P;
@@ -700,8 +742,8 @@ int32_t pyomgpu_precond_train_step(pyomgpu_precond* P, const double* r, const do
   if (run_net(P, st)) return pfail(PYOMGPU_ECUDA, "train_step: forward launch failed");
   const size_t npx = (size_t)P->Hp * P->Wp;
   k_loss_fields<<<nb, kRB, 0, st>>>(g, P->net.z, e, P->stat, P->Wp, P->sc, P->nu, P->dbar, P->w1, P->w2);
-  k_loss_dots<<<nb, kRB, 0, st>>>(g, c->sf.dev(), P->w1, P->w2, c->dxu, c->dyu, c->cosu, P->t1, P->t2, P->part);
-  k_loss_scalars<<<1, 32, 0, st>>>(P->part, nb, P->sc);
+  k_loss_dots<<<nb, kRB, 0, st>>>(g, c->sf.dev(), P->w1, P->w2, c->dxu, c->dyu, c->cosu, P->t1, P->t2, P->part,
+                                  P->arrived, P->sc);
   k_loss_grad<<<blocks_for(npx), kRB, 0, st>>>(g, P->t1, P->t2, P->stat, P->Hp, P->Wp, P->sc, P->gz);
   if (unet_backward(P->net, P->gz, st)) return pfail(PYOMGPU_ECUDA, "train_step: backward launch failed");
   if (lr > 0.f) unet_adam(P->net, lr, st);
@@ -741,10 +783,9 @@ int32_t pyomgpu_solve_fcg(pyomgpu_ctx* c, pyomgpu_precond* P, const double* forc
   for (double* a : {P->p1, P->p2, P->ap1, P->ap2}) cudaMemsetAsync(a, 0, g.size() * sizeof(double), st);
   k_set_scalar<<<1, 1, 0, st>>>(P->sc, kRtol2BB, rtol * rtol);
   k_set_scalar<<<1, 1, 0, st>>>(P->sc, kMaxIt, (double)max_it);
-  k_residual_vec<<<nb, kRB, 0, st>>>(g, c->sf.dev(), f, c->sol, P->r, P->part);
-  k_scalars<<<1, 32, 0, st>>>(P->part, nb, 0, P->sc);
+  k_residual_vec<<<nb, kRB, 0, st>>>(g, c->sf.dev(), f, c->sol, P->r, P->part, P->arrived, P->sc);
   cudaMemsetAsync(P->net.err, 0, sizeof(int), st);
-  int launches = 5;
+  int launches = 4;
   // the captured iteration runs on its own stream: order it after st
   cudaEvent_t ev = nullptr;
   cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
