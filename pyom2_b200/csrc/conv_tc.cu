@@ -57,12 +57,15 @@ struct ConvShape {
   static constexpr int CW = COUT / 2;  // channels per warpgroup
 };
 
-__device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 __device__ __forceinline__ uint16_t f2bf(float f) {
   __nv_bfloat16 h = __float2bfloat16_rn(f);
   return *reinterpret_cast<uint16_t*>(&h);
 }
-__device__ __forceinline__ uint32_t pack2(float a, float b) { return (uint32_t)f2bf(a) | ((uint32_t)f2bf(b) << 16); }
+// two values rounded to nearest even in one conversion, a in the low half
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
 __device__ __forceinline__ uint4 pack8(const float* r) {
   uint4 o;
   o.x = pack2(r[0], r[1]);
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
   const uint32_t sw_addr = smem_u32(sw);
   constexpr uint32_t kIdesc = tc::idesc_bf16_f32(128, COUT);
   constexpr uint32_t kPlane = (uint32_t)S::BH * kBW * 16;  // bytes between channel groups of the box
+  const uint64_t bd0 = tc::smem_desc(sw_addr, COUT * 16, 128);
 
   int it = 0;
   for (int tile = blockIdx.x; ok && tile < a.ntiles; tile += gridDim.x, ++it) {
@@ -170,24 +174,21 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
       // buffer b^1 was read by the MMAs of the previous tile, which completed
       if (next < a.ntiles) issue_tile(next, b ^ 1);
       tc::fence_after_sync();
-      const uint32_t sx_addr = smem_u32(base + b * S::XSTRIDE);
-#pragma unroll 1
-      for (int t = 0; t < ROWS; t++) {
-        uint32_t acc = 0;
-#pragma unroll 1
-        for (int tap = 0; tap < 9; tap++) {
-          const int dy = tap / 3, dx = tap - 3 * (tap / 3);
+      // Descriptors as one base plus constants (an address field of 14 bits holds every offset without a carry),
+      // unrolled: built per MMA by this one thread they took ~90 to 150 cycles each, more than the MMA itself
+      // (5300 to 7600 of ~10000 cycles a tile).
+      const uint64_t ad0 = tc::smem_desc(smem_u32(base + b * S::XSTRIDE), kPlane, 128);
+#pragma unroll
+      for (int t = 0; t < ROWS; t++)
+#pragma unroll
+        for (int tap = 0; tap < 9; tap++)
 #pragma unroll
           for (int k = 0; k < CIN / 16; k++) {
-            const uint32_t aaddr = sx_addr + (uint32_t)(2 * k) * kPlane + (uint32_t)((t + dy) * kBW + dx) * 16u;
-            const uint32_t baddr = sw_addr + (uint32_t)((tap * S::GIN + 2 * k) * COUT) * 16u;
-            const uint64_t ad = tc::smem_desc(aaddr, kPlane, 128);
-            const uint64_t bd = tc::smem_desc(baddr, COUT * 16, 128);
-            tc::mma_bf16(tmem + (uint32_t)(t * COUT), ad, bd, kIdesc, acc);
-            acc = 1;
+            const uint32_t ao = (uint32_t)(2 * k) * kPlane + (uint32_t)((t + tap / 3) * kBW + tap % 3) * 16u;
+            const uint32_t bo = (uint32_t)((tap * S::GIN + 2 * k) * COUT) * 16u;
+            tc::mma_bf16(tmem + (uint32_t)(t * COUT), ad0 + (ao >> 4), bd0 + (bo >> 4), kIdesc,
+                         tap == 0 && k == 0 ? 0u : 1u);
           }
-        }
-      }
       tc::commit(bar_mma);
     }
     if (next < a.ntiles) pend_buf = b ^ 1;
@@ -202,42 +203,54 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
     const int x = x0 + 32 * quarter + lane;
     const bool in_x = 32 * quarter + lane < kConvTileX && x < a.W;  // the last two rows of M are the rim's
     const uint32_t trow = tmem + ((uint32_t)(32 * quarter) << 16);
+    // The operands from global memory (skip, gate) of a group of channels are fetched before its accumulators are
+    // waited for, and before any store, so their latencies overlap.
 #pragma unroll 1
     for (int t = 0; t < ROWS; t += 2) {
       const int ya = y0 + t, yb = ya + 1;
-#pragma unroll 1
-      for (int c0 = half * S::CW; c0 < (half + 1) * S::CW; c0 += 8) {
+      const bool in_a = in_x && ya < a.H, in_b = in_x && yb < a.H;
+      if (a.epi == kEpiF32) {  // channel 0 only
+        if (half == 0) {
+          float r0[8], r1[8];
+          tmem_ld8(trow + (uint32_t)(t * COUT), r0);
+          tmem_ld8(trow + (uint32_t)((t + 1) * COUT), r1);
+          tc::wait_ld();
+          float* y32 = reinterpret_cast<float*>(a.y);
+          if (in_a) y32[(size_t)ya * a.W + x] = r0[0] + sbias[0];
+          if (in_b) y32[(size_t)yb * a.W + x] = r1[0] + sbias[0];
+        }
+        continue;
+      }
+      constexpr int kGroups = S::CW / 8;
+#pragma unroll(kGroups > 2 ? 2 : kGroups)
+      for (int gi = 0; gi < kGroups; gi++) {
+        const int c0 = half * S::CW + 8 * gi, g = c0 >> 3;
         float r0[8], r1[8];
         tmem_ld8(trow + (uint32_t)(t * COUT + c0), r0);
         tmem_ld8(trow + (uint32_t)((t + 1) * COUT + c0), r1);
-        tc::wait_ld();
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          r0[k] += sbias[c0 + k];
-          r1[k] += sbias[c0 + k];
-        }
-        if (a.epi == kEpiF32) {
-          if (c0 == 0 && in_x) {
-            float* y32 = reinterpret_cast<float*>(a.y);
-            if (ya < a.H) y32[(size_t)ya * a.W + x] = r0[0];
-            if (yb < a.H) y32[(size_t)yb * a.W + x] = r1[0];
-          }
-          continue;
-        }
-        const int g = c0 >> 3;
         if (a.epi == kEpiPlain) {
-          float p[8];
-#pragma unroll
-          for (int k = 0; k < 8; k++) p[k] = 0.f;
+          const size_t off = (((size_t)g * a.H + ya) * a.W + x) * 8, offb = off + (size_t)a.W * 8;
+          const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+          uint4 add0 = zero, add1 = zero, gt0 = zero, gt1 = zero;
+          if (a.addend) {
+            if (in_a) add0 = __ldg(reinterpret_cast<const uint4*>(a.addend + off));
+            if (in_b) add1 = __ldg(reinterpret_cast<const uint4*>(a.addend + offb));
+          }
+          if (a.gate) {
+            if (in_a) gt0 = __ldg(reinterpret_cast<const uint4*>(a.gate + off));
+            if (in_b) gt1 = __ldg(reinterpret_cast<const uint4*>(a.gate + offb));
+          }
+          tc::wait_ld();
+          uint4 o[2];
 #pragma unroll
           for (int rr = 0; rr < 2; rr++) {
             float* r = rr ? r1 : r0;
-            const int yy = rr ? yb : ya;
-            const bool in = in_x && yy < a.H;
-            const size_t off = (((size_t)g * a.H + yy) * a.W + x) * 8;
+#pragma unroll
+            for (int k = 0; k < 8; k++) r[k] += sbias[c0 + k];
+            const bool in = rr ? in_b : in_a;
             if (a.addend && in) {
               float q[8];
-              unpack8(*reinterpret_cast<const uint4*>(a.addend + off), q);
+              unpack8(rr ? add1 : add0, q);
 #pragma unroll
               for (int k = 0; k < 8; k++) r[k] += q[k];
             }
@@ -247,50 +260,60 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
             }
             if (a.gate && in) {
               float q[8];
-              unpack8(*reinterpret_cast<const uint4*>(a.gate + off), q);
+              unpack8(rr ? gt1 : gt0, q);
 #pragma unroll
               for (int k = 0; k < 8; k++) r[k] = q[k] > 0.f ? r[k] : 0.f;
             }
-            if (in) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.y) + off) = pack8(r);
-#pragma unroll
-            for (int k = 0; k < 8; k++) p[k] += bf2f(f2bf(r[k]));  // pool what was stored
+            o[rr] = pack8(r);
+            if (in) *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.y) + (rr ? offb : off)) = o[rr];
           }
-          if (a.pool_out) {  // 2x2 average: rows ya, yb in this thread, columns x, x^1 in lanes l, l^1
+          if (a.pool_out) {  // 2x2 average of what was stored: rows ya, yb here, columns x, x^1 in lanes l, l^1
+            float p[8], q[8];
+            unpack8(o[0], p);
+            unpack8(o[1], q);
 #pragma unroll
-            for (int k = 0; k < 8; k++) p[k] = 0.25f * (p[k] + __shfl_xor_sync(0xffffffffu, p[k], 1));
-            if ((lane & 1) == 0 && in_x && ya < a.H) {
+            for (int k = 0; k < 8; k++) {
+              p[k] = (0.f + p[k]) + q[k];
+              p[k] = 0.25f * (p[k] + __shfl_xor_sync(0xffffffffu, p[k], 1));
+            }
+            if ((lane & 1) == 0 && in_a) {
               const int H2 = a.H >> 1, W2 = a.W >> 1;
               *reinterpret_cast<uint4*>(a.pool_out + (((size_t)g * H2 + (ya >> 1)) * W2 + (x >> 1)) * 8) = pack8(p);
             }
           }
         } else {  // kEpiUp: every coarse pixel feeds its 2x2 fine block
           const int H2 = 2 * a.H, W2 = 2 * a.W;
+          const size_t off = (((size_t)g * H2 + 2 * ya) * W2 + 2 * x) * 8;
+          const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+          uint4 s2[4][2];  // fine rows 2 ya .. 2 yb + 1
+#pragma unroll
+          for (int f = 0; f < 4; f++) {
+            const uint4* src = reinterpret_cast<const uint4*>(a.addend + off + (size_t)f * W2 * 8);
+            const bool in = f < 2 ? in_a : in_b;
+            s2[f][0] = in ? __ldg(src) : zero;
+            s2[f][1] = in ? __ldg(src + 1) : zero;
+          }
+          tc::wait_ld();
 #pragma unroll
           for (int rr = 0; rr < 2; rr++) {
-            const float* r = rr ? r1 : r0;
-            const int yy = rr ? yb : ya;
-            if (!(in_x && yy < a.H)) continue;
+            float* r = rr ? r1 : r0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) r[k] += sbias[c0 + k];
+            if (!(rr ? in_b : in_a)) continue;
 #pragma unroll
             for (int fy = 0; fy < 2; fy++) {
-              const size_t off = (((size_t)g * H2 + 2 * yy + fy) * W2 + 2 * x) * 8;
-              uint4 s2[2];
-              s2[0] = *reinterpret_cast<const uint4*>(a.addend + off);
-              s2[1] = *reinterpret_cast<const uint4*>(a.addend + off + 8);
-              uint4 o2[2];
+              uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.y) + off + (size_t)(2 * rr + fy) * W2 * 8);
 #pragma unroll
               for (int fx = 0; fx < 2; fx++) {
-                float s[8];
-                unpack8(s2[fx], s);
+                float v[8];
+                unpack8(s2[2 * rr + fy][fx], v);
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
-                  s[k] += r[k];
-                  if (a.relu) s[k] = fmaxf(s[k], 0.f);
+                  v[k] += r[k];
+                  if (a.relu) v[k] = fmaxf(v[k], 0.f);
                 }
-                o2[fx] = pack8(s);
+                dst[fx] = pack8(v);
               }
-              uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.y) + off);
-              dst[0] = o2[0];
-              dst[1] = o2[1];
             }
           }
         }
