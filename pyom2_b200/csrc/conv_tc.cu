@@ -3,8 +3,8 @@
 // One CTA (8 warps) walks output tiles of ROWS rows x 126 pixels.  Per tile
 // one TMA load brings the (ROWS+2) x 128 x Cin input box (zero-filled outside
 // the image = the convolution's zero padding) into shared memory; thread 0
-// issues 9 taps x Cin/16 MMAs of M=128, N=Cout, K=16 per output row, each A
-// operand being the box shifted by the tap offset; the accumulators
+// issues 3 x Cin/16 MMAs of M=128, K=16 per box row, each A operand being the
+// box row shifted by dx and N = Cout times the output rows it feeds; the accumulators
 // (ROWS x Cout f32 columns) live in TMEM.  The 8 warps read them back for
 // the fused epilogue: warp w owns TMEM lane quarter w % 4 (32 output
 // pixels) and channel half w / 4.
@@ -12,8 +12,7 @@
 // Schedule: the packed weights (one bulk copy) and the first input box are
 // requested together; input boxes are double-buffered, so the load of the
 // next tile runs under the MMAs and the epilogue of the current one.  ROWS is
-// 4, or 2 when Cin = 64 (two 64-channel boxes and the weights then still fit
-// in shared memory, and small coarse-level images get more CTAs).
+// 4, 2 or 1 (launch_one).
 //
 // Waits on the mbarriers are bounded by %globaltimer; on time-out the kernel
 // records PYOMGPU_TIMEOUT, waits (bounded) for the copies and MMAs it issued,
@@ -41,9 +40,8 @@ __host__ __device__ constexpr uint32_t pow2_cols(uint32_t n) {
   return c;
 }
 
-template <int CIN, int COUT>
+template <int CIN, int COUT, int ROWS>
 struct ConvShape {
-  static constexpr int ROWS = CIN == 64 ? 2 : 4;
   static constexpr int BH = ROWS + 2;
   static constexpr int GIN = CIN / 8;
   static constexpr uint32_t XBYTES = (uint32_t)GIN * BH * kBW * 16;
@@ -100,10 +98,9 @@ __device__ __forceinline__ bool cta_wait(uint64_t* bar, uint32_t parity, unsigne
   return __syncthreads_and(mbar_wait_bounded(bar, parity, timeout_ns)) != 0;
 }
 
-template <int CIN, int COUT>
+template <int CIN, int COUT, int ROWS>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_constant__ ConvArgs a) {
-  using S = ConvShape<CIN, COUT>;
-  constexpr int ROWS = S::ROWS;
+  using S = ConvShape<CIN, COUT, ROWS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sw = base + S::WOFF;
@@ -154,9 +151,8 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
   }
 
   const uint32_t sw_addr = smem_u32(sw);
-  constexpr uint32_t kIdesc = tc::idesc_bf16_f32(128, COUT);
   constexpr uint32_t kPlane = (uint32_t)S::BH * kBW * 16;  // bytes between channel groups of the box
-  const uint64_t bd0 = tc::smem_desc(sw_addr, COUT * 16, 128);
+  const uint64_t bd0 = tc::smem_desc(sw_addr, 3 * COUT * 16, 128);
 
   int it = 0;
   for (int tile = blockIdx.x; ok && tile < a.ntiles; tile += gridDim.x, ++it) {
@@ -177,18 +173,30 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
       // Descriptors as one base plus constants (an address field of 14 bits holds every offset without a carry),
       // unrolled: built per MMA by this one thread they took ~90 to 150 cycles each, more than the MMA itself
       // (5300 to 7600 of ~10000 cycles a tile).
+      // An MMA takes ~58 cycles for its 128 pixel rows of A however few channels it multiplies them with, so a box
+      // row y is multiplied once per dx with the weights of all the output rows t = y-2 .. y it belongs to
+      // (dy = y - t), which sit side by side in N as their accumulators do in TMEM; the first product of row t = y
+      // is its own MMA, as it starts from zero.  Every output still sums its products in the order dy, dx, k.
       const uint64_t ad0 = tc::smem_desc(smem_u32(base + b * S::XSTRIDE), kPlane, 128);
 #pragma unroll
-      for (int t = 0; t < ROWS; t++)
+      for (int y = 0; y < ROWS + 2; y++) {
+        const int t0 = y > 2 ? y - 2 : 0, t1 = y < ROWS ? y : ROWS - 1;
 #pragma unroll
-        for (int tap = 0; tap < 9; tap++)
+        for (int dx = 0; dx < 3; dx++)
 #pragma unroll
           for (int k = 0; k < CIN / 16; k++) {
-            const uint32_t ao = (uint32_t)(2 * k) * kPlane + (uint32_t)((t + tap / 3) * kBW + tap % 3) * 16u;
-            const uint32_t bo = (uint32_t)((tap * S::GIN + 2 * k) * COUT) * 16u;
-            tc::mma_bf16(tmem + (uint32_t)(t * COUT), ad0 + (ao >> 4), bd0 + (bo >> 4), kIdesc,
-                         tap == 0 && k == 0 ? 0u : 1u);
+            const uint64_t ad = ad0 + (((uint32_t)(2 * k) * kPlane + (uint32_t)(y * kBW + dx) * 16u) >> 4);
+            const uint64_t bd = bd0 + (uint32_t)((dx * S::GIN + 2 * k) * 3 * COUT);  // in 16-byte units
+            const bool first = dx == 0 && k == 0 && y < ROWS;
+            const int n = (first ? y : t1 + 1) - t0;  // output rows that go on accumulating
+            if (n > 0)
+              tc::mma_bf16(tmem + (uint32_t)(t0 * COUT), ad, bd + (uint32_t)((t0 - y + 2) * COUT),
+                           tc::idesc_bf16_f32(128, n * COUT), 1u);
+            if (first)
+              tc::mma_bf16(tmem + (uint32_t)(y * COUT), ad, bd + (uint32_t)(2 * COUT),
+                           tc::idesc_bf16_f32(128, COUT), 0u);
           }
+      }
       tc::commit(bar_mma);
     }
     if (next < a.ntiles) pend_buf = b ^ 1;
@@ -208,12 +216,12 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
 #pragma unroll 1
     for (int t = 0; t < ROWS; t += 2) {
       const int ya = y0 + t, yb = ya + 1;
-      const bool in_a = in_x && ya < a.H, in_b = in_x && yb < a.H;
+      const bool in_a = in_x && ya < a.H, in_b = ROWS > 1 && in_x && yb < a.H;
       if (a.epi == kEpiF32) {  // channel 0 only
         if (half == 0) {
           float r0[8], r1[8];
           tmem_ld8(trow + (uint32_t)(t * COUT), r0);
-          tmem_ld8(trow + (uint32_t)((t + 1) * COUT), r1);
+          tmem_ld8(trow + (uint32_t)((ROWS > 1 ? t + 1 : t) * COUT), r1);
           tc::wait_ld();
           float* y32 = reinterpret_cast<float*>(a.y);
           if (in_a) y32[(size_t)ya * a.W + x] = r0[0] + sbias[0];
@@ -227,7 +235,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
         const int c0 = half * S::CW + 8 * gi, g = c0 >> 3;
         float r0[8], r1[8];
         tmem_ld8(trow + (uint32_t)(t * COUT + c0), r0);
-        tmem_ld8(trow + (uint32_t)((t + 1) * COUT + c0), r1);
+        tmem_ld8(trow + (uint32_t)((ROWS > 1 ? t + 1 : t) * COUT + c0), r1);
         if (a.epi == kEpiPlain) {
           const size_t off = (((size_t)g * a.H + ya) * a.W + x) * 8, offb = off + (size_t)a.W * 8;
           const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -337,24 +345,26 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
 
 // ---------------------------------------------------------------- weights
 __global__ void k_pack_weights(const float* __restrict__ w, int cout, int cin, int flip, uint16_t* __restrict__ out) {
-  // forward: out[tap][ci/8][co][ci%8] = w[co][ci][tap]
-  // flip:    out[tap][co/8][ci][co%8] = w[co][ci][8-tap]   (input channels = forward cout)
+  // out[dx][ci/8][2-dy][co][ci%8] = w[co][ci][3 dy + dx]; flip: input channels = forward cout, taps rotated
+  // (dx -> 2-dx, dy -> 2-dy).  The three dy of a dx are neighbours in N, in the order of the output rows they
+  // feed.
   const int n = 9 * cin * cout;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int co = e / (cin * 9), rem = e - co * cin * 9, ci = rem / 9, tap = rem - ci * 9;
+    const int dy = tap / 3, dx = tap - 3 * dy;
     const float v = w[e];
     size_t o;
     if (!flip)
-      o = (((size_t)tap * (cin / 8) + ci / 8) * cout + co) * 8 + (ci & 7);
+      o = (((size_t)(dx * (cin / 8) + ci / 8) * 3 + (2 - dy)) * cout + co) * 8 + (ci & 7);
     else
-      o = (((size_t)(8 - tap) * (cout / 8) + co / 8) * cin + ci) * 8 + (co & 7);
+      o = (((size_t)((2 - dx) * (cout / 8) + co / 8) * 3 + dy) * cin + ci) * 8 + (co & 7);
     out[o] = f2bf(v);
   }
 }
 
-template <int CIN, int COUT>
-int launch_one(const ConvSpec& s, int nsm, cudaStream_t st) {
-  using S = ConvShape<CIN, COUT>;
+template <int CIN, int COUT, int ROWS>
+int launch_rows(const ConvSpec& s, int nsm, cudaStream_t st) {
+  using S = ConvShape<CIN, COUT, ROWS>;
   // Shared memory requested so that no more CTAs fit on an SM than its 512
   // TMEM columns hold (an allocation beyond them would wait for a CTA to exit).
   constexpr uint32_t kTmemCtas = 512u / S::NCOLS;
@@ -362,7 +372,7 @@ int launch_one(const ConvSpec& s, int nsm, cudaStream_t st) {
   static_assert(kSmemReq <= 232448u, "shared memory of one CTA");
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kSmemReq);
     if (e != cudaSuccess) return (int)e;
     attr = true;
@@ -384,7 +394,7 @@ int launch_one(const ConvSpec& s, int nsm, cudaStream_t st) {
   a.H = s.H;
   a.W = s.W;
   a.tiles_x = (s.W + kConvTileX - 1) / kConvTileX;
-  a.ntiles = a.tiles_x * ((s.H + S::ROWS - 1) / S::ROWS);
+  a.ntiles = a.tiles_x * ((s.H + ROWS - 1) / ROWS);
   a.relu = s.relu;
   a.epi = s.epi;
   a.err = s.err;
@@ -392,8 +402,21 @@ int launch_one(const ConvSpec& s, int nsm, cudaStream_t st) {
   int per_sm = (int)std::min<uint32_t>(233472u / kSmemReq, kTmemCtas);
   if (per_sm < 1) per_sm = 1;
   const int grid = std::max(1, std::min(a.ntiles, per_sm * nsm));
-  conv3x3_tc_kernel<CIN, COUT><<<grid, kConvThreads, kSmemReq, st>>>(a);
+  conv3x3_tc_kernel<CIN, COUT, ROWS><<<grid, kConvThreads, kSmemReq, st>>>(a);
   return (int)cudaGetLastError();
+}
+
+// Tile height: 4 rows, or 2 with 64 input channels (two boxes and the weights
+// then fit in shared memory).  Coarse levels have fewer tiles than SMs (23 of
+// 64 channels at 90 x 45); they take half the height, so that a tile's MMAs and
+// epilogue, which nothing else overlaps there, take half the time.  The pool
+// needs row pairs.
+template <int CIN, int COUT>
+int launch_one(const ConvSpec& s, int nsm, cudaStream_t st) {
+  constexpr int kRows = CIN == 64 ? 2 : 4;
+  const int tiles = ((s.W + kConvTileX - 1) / kConvTileX) * ((s.H + kRows - 1) / kRows);
+  if (tiles < nsm && (!s.pool_out || kRows > 2)) return launch_rows<CIN, COUT, kRows / 2>(s, nsm, st);
+  return launch_rows<CIN, COUT, kRows>(s, nsm, st);
 }
 
 }  // namespace

@@ -32,7 +32,7 @@ enum ConvEpilogue : int { kEpiPlain = 0, kEpiUp = 1, kEpiF32 = 2 };
 
 struct ConvArgs {
   CUtensorMap map_x;      // input, box (2 x 128 64-bit words, rows+2, Cin/8), rows = the instantiation's tile height
-  const uint16_t* wpack;  // [9][Cin/8][Cout][8] bf16
+  const uint16_t* wpack;  // [dx][Cin/8][2-dy][Cout][8] bf16
   const float* bias;      // [Cout] or null
   void* y;
   const uint16_t* gate;
@@ -69,7 +69,7 @@ bool conv3x3_supported(int cin, int cout);
 int conv3x3_dw_launch(int cin, int cout, const uint16_t* X, const uint16_t* G, int H, int W, float* dW, float* db,
                       int nsm, int* err, unsigned long long timeout_ns, cudaStream_t st);
 
-// Packs f32 weights [Cout][Cin][3][3] into [tap][Cin/8][Cout][8] bf16 (round
+// Packs f32 weights [Cout][Cin][3][3] into [dx][Cin/8][2-dy][Cout][8] bf16 (round
 // to nearest even).  flip packs the backward-data kernel instead: channels
 // transposed and taps rotated by 180 degrees (its input channels are the
 // forward Cout).
