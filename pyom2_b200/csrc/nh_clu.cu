@@ -14,7 +14,7 @@
 // The kernel it replaces for these sizes (one cell per thread in compact order,
 // neighbours read from the owners' shared memory in both sweeps, two cluster
 // barriers and two 32-warp reductions an iteration) took 7.06 us per iteration
-// on a 160 x 1 x 60 slice.
+// on a 160 x 1 x 60 slice; this one 3.10 us.
 #include <math.h>
 
 #include "cg_clu.cuh"
@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(NT, 1) nh_clu_kernel(const __grid_constant__ N
   const double tE = nlev > 0 ? op.tE[q2] : 0.0, tW = nlev > 0 ? op.tW[q2] : 0.0;
   const double tN = nlev > 0 ? op.tN[j + 1] : 0.0, tS = nlev > 0 ? op.tS[j + 1] : 0.0;
   double s[P], q[P], r[P], x[P];  // direction, A s, residual, p_non_hydro
+  double cc[P];                   // centre coefficient, in make_coeff_non_hydro's accumulation order
   uint32_t fl[(P + 3) / 4];       // flag bytes
   auto flag = [&](int u) -> uint32_t { return fl[u / 4] >> (8 * (u % 4)) & 0xffu; };
 
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(NT, 1) nh_clu_kernel(const __grid_constant__ N
     face(2 * nWE + nSN, pw, (ph + 1) * sp + 1, 1, rN);
   };
 
+  bool ns = false;  // a cell of this warp has a south or a north face (an x-z slice has none)
   int how = NHCtl::kGo;
   // ------------------------------------------------------------------ init
   // res = forc - A p (interior), rsold = dot_3D(res, res)  (:163-176)
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(NT, 1) nh_clu_kernel(const __grid_constant__ N
     for (int w = 0; w < (P + 3) / 4; w++) fl[w] = 0;
 #pragma unroll
     for (int u = 0; u < P; u++) {
-      s[u] = q[u] = r[u] = x[u] = 0.0;
+      s[u] = q[u] = r[u] = x[u] = cc[u] = 0.0;
       if (u < nlev) {
         const int k = k0 + u + 1;
         const size_t c = G.at(i, j, k);
@@ -165,12 +167,17 @@ __global__ void __launch_bounds__(NT, 1) nh_clu_kernel(const __grid_constant__ N
         r[u] = __dsub_rn(fo, a);
         x[u] = Pm.p[c];
         fl[u / 4] |= f << (8 * (u % 4));
+        cc[u] = nh_centre(f, tE, tW, tN, tS, stT[k0 + u], stT[kp + k0 + u]);
         if (f & kNHMaskT) {
           v[0] += r[u] * r[u];
           v[1] += fo * fo;
         }
       }
     }
+    uint32_t any = 0;
+#pragma unroll
+    for (int w = 0; w < (P + 3) / 4; w++) any |= fl[w];
+    ns = __any_sync(0xffffffffu, any & (kNHN | kNHS) * 0x01010101u);
     stage();
     clu_sync();  // every inbox is cleared, the faces staged
     send_halo(xch);
@@ -196,16 +203,32 @@ __global__ void __launch_bounds__(NT, 1) nh_clu_kernel(const __grid_constant__ N
     if (nlev > 0) {
       const double* o = ss + (k0 + 1) * lv + (ly + 1) * sp + lx + 1;
       const double below = o[-lv], above = o[nlev * lv];
+      // nh_row term by term over the segment, with selects and the centre coefficient kept: its tests as branches
+      // ran one level after the other (8 levels a thread: 240 x 1 x 80 in 4.76 us per iteration, now 3.99; one
+      // block, 64 x 1 x 24: 2.52, now 1.69; 160 x 1 x 60 with 4 levels: 3.20, now 3.10)
+      auto term = [&](uint32_t face, auto coef, auto val) {
+#pragma unroll
+        for (int u = 0; u < P; u++) {  // no face beyond the segment's last level: A s = 0 there
+          const double n = __dadd_rn(q[u], __dmul_rn(coef(u), val(u)));
+          q[u] = (flag(u) & face) ? n : q[u];
+        }
+      };
+#pragma unroll
+      for (int u = 0; u < P; u++) q[u] = 0.0;
+      term(kNHB, [&](int u) { return stT[kp + k0 + u]; }, [&](int u) { return u > 0 ? s[u > 0 ? u - 1 : 0] : below; });
+      if (ns) term(kNHS, [&](int) { return tS; }, [&](int u) { return o[u * lv - sp]; });
+      term(kNHW, [&](int) { return tW; }, [&](int u) { return o[u * lv - 1]; });
+#pragma unroll
+      for (int u = 0; u < P; u++) q[u] = __dadd_rn(q[u], __dmul_rn(cc[u], s[u]));
+      term(kNHE, [&](int) { return tE; }, [&](int u) { return o[u * lv + 1]; });
+      if (ns) term(kNHN, [&](int) { return tN; }, [&](int u) { return o[u * lv + sp]; });
+      term(kNHT, [&](int u) { return stT[k0 + u]; },
+           [&](int u) { return u + 1 == nlev ? above : s[u + 1 < P ? u + 1 : u]; });
 #pragma unroll
       for (int u = 0; u < P; u++) {
-        const uint32_t f = flag(u);  // no face beyond the segment's last level: A s = 0 there
-        const double up = u + 1 == nlev ? above : s[u + 1 < P ? u + 1 : u], dn = u > 0 ? s[u > 0 ? u - 1 : 0] : below;
-        const double a = nh_row(f, tE, tW, tN, tS, stT[k0 + u], stT[kp + k0 + u], dn, o[u * lv - sp], o[u * lv - 1],
-                                s[u], o[u * lv + 1], o[u * lv + sp], up);
-        const bool wet = f & kNHMaskT;
-        vA[0] += wet ? s[u] * a : 0.0;
+        const bool wet = flag(u) & kNHMaskT;
+        vA[0] += wet ? s[u] * q[u] : 0.0;
         vA[1] = fmax(vA[1], wet ? fabs(s[u]) : 0.0);
-        q[u] = a;
       }
     }
     ++ep;

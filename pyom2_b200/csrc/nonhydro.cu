@@ -1078,12 +1078,26 @@ void nh_clu_config(const NHCut& c, cudaLaunchConfig_t& cfg, cudaLaunchAttribute&
   cfg.numAttrs = 1;
 }
 
-// Estimated iteration time (ns) of the cluster kernel on nb pieces of w x h
-// columns with nt threads of p levels.
-double nh_clu_iter_ns(int w, int h, int nz, int p, int nt, int nb) {
-  const double faces = nb == 1 ? 0.0 : 2.0 * (w + h) * nz / nt;  // records a thread sends and receives
-  if (nb == 1) return nt == 128 ? 900.0 + 90.0 * p : 1000.0 + 150.0 * p;
-  return 60.0 * faces + (nt == 128 ? 1050.0 + 130.0 * p + 20.0 * nb : 1100.0 + 180.0 * p + 42.0 * nb);
+// Estimated iteration time (ns) of the cluster kernel on npx x npy pieces of
+// at most w x h columns with nt threads of p levels: a block's own work, its
+// passes over the faces it exchanges, their records.  Within ~10 % of the times
+// of 60 cuts (us per iteration; threads/levels): 64 x 1 x 64 128/4 on 8, 12
+// (unequal pieces), 16 blocks 2.50, 2.72, 2.58; 160 x 1 x 60 256/4 on 10, 16
+// 3.10, 3.17, 128/8 on 16 3.37; 240 x 1 x 80 256/8 on 12, 15 3.99, 4.18,
+// 256/12 on 16 5.53; 64 x 1 x 24 one block 256/8 1.69, two of 256/4 2.41;
+// 40 x 24 x 10 256/4 on 6 x 2, 4 x 3 3.73, 4.03; 40 x 36 x 9 256/8 on 2 x 6,
+// 4 x 3, 14 x 1 4.67, 5.08, 5.72; 48 x 40 x 24 256/12 on 8 x 2, 16 x 1 9.06,
+// 11.42.
+double nh_clu_iter_ns(const pyomgpu_nh* h, int npx, int npy, int w, int hh, int p, int nt) {
+  const int nz = h->G.nz, nb = npx * npy;
+  if (nb == 1) return 1000.0 + 85.0 * p;
+  auto sides = [](int n, bool cyclic) { return n > 2 || cyclic ? 2 : n - 1; };  // faces of a block along one direction
+  const int we = sides(npx, h->cyclic_x), sn = sides(npy, h->cyclic_y);
+  const int passes = we * ((hh * nz + nt - 1) / nt) + sn * ((w * nz + nt - 1) / nt);
+  const double records = (double)(we * hh + sn * w) * nz / nt;  // a thread
+  const bool unequal = h->G.g.nx % npx != 0 || h->G.g.ny % npy != 0;
+  return (nt == 128 ? 1300.0 + 20.0 * nb : 1800.0 + 30.0 * nb) + (p == 4 ? 0.0 : p == 8 ? 900.0 : 2600.0) +
+         400.0 * passes + 350.0 * records + (unequal ? 100.0 : 0.0);
 }
 
 // Cut of the grid for the cluster kernel (nh_clu.cu), planned once: among the
@@ -1105,7 +1119,7 @@ bool nh_clu_plan(pyomgpu_nh* h) {
         const int nt = np[0], p = np[1];
         const size_t smem = nh_clu_smem_bytes(w, hh, nz, p);
         if (smem > kNHSmallSmemMax || (size_t)w * hh * ((nz + p - 1) / p) > (size_t)nt) continue;
-        const double c = nh_clu_iter_ns(w, hh, nz, p, nt, npx * npy);
+        const double c = nh_clu_iter_ns(h, npx, npy, w, hh, p, nt);
         if (c < cost) {
           cost = c;
           best = NHCut{npx, npy, w, hh, p, nt, smem};

@@ -60,18 +60,23 @@ struct NHOp {
   }
 };
 
-// Operator row with the seven field values given: bottom, south, west,
-// centre, east, north, top; t* are the face factors (read only where the
-// face flag is set).
-__device__ __forceinline__ double nh_row(uint32_t f, double tE, double tW, double tN, double tS, double tT, double tB,
-                                         double vb, double vs, double vw, double vc, double ve, double vn, double vt) {
-  double c = 0.0;  // make_coeff_non_hydro's accumulation order
+// Centre coefficient of a cell's row (make_coeff_non_hydro's accumulation order).
+__device__ __forceinline__ double nh_centre(uint32_t f, double tE, double tW, double tN, double tS, double tT, double tB) {
+  double c = 0.0;
   if (f & kNHE) c = __dsub_rn(c, tE);
   if (f & kNHW) c = __dsub_rn(c, tW);
   if (f & kNHN) c = __dsub_rn(c, tN);
   if (f & kNHS) c = __dsub_rn(c, tS);
   if (f & kNHT) c = __dsub_rn(c, tT);
   if (f & kNHB) c = __dsub_rn(c, tB);
+  return c;
+}
+// Operator row with the seven field values given: bottom, south, west,
+// centre, east, north, top; t* are the face factors (read only where the
+// face flag is set).
+__device__ __forceinline__ double nh_row(uint32_t f, double tE, double tW, double tN, double tS, double tT, double tB,
+                                         double vb, double vs, double vw, double vc, double ve, double vn, double vt) {
+  const double c = nh_centre(f, tE, tW, tN, tS, tT, tB);
   // apply_op_3D: kk outermost, then jj, then ii; zero coefficients add nothing
   double a = 0.0;
   if (f & kNHB) a = __dadd_rn(a, __dmul_rn(tB, vb));

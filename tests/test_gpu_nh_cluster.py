@@ -1,0 +1,59 @@
+"""Small non-hydrostatic grids in one thread-block cluster (nh_clu.cu): the automatic kernel choice
+against the oracle, from one block of a few cells to the largest cluster and beyond it; and the
+warp-uniform fast paths of the brick kernel (all faces, none, mixed) on the same problems."""
+import warnings
+
+import numpy as np
+import pytest
+
+from pyom2_b200 import synth
+from pyom2_b200.model import ModelState
+from pyom2_b200.non_hydrostatic import NonHydrostatic
+
+pytestmark = pytest.mark.gpu
+
+
+def tank(nx, ny, nz, cyc_x, cyc_y):
+    rng = np.random.default_rng(nx + 31 * ny + 977 * nz)
+    M = ModelState(nx, ny, nz, enable_cyclic_x=cyc_x, enable_cyclic_y=cyc_y, coord_degree=False)
+    M.dxt[2:nx + 2] = 0.01
+    M.dyt[2:ny + 2] = 0.012
+    M.dzt[:] = 0.011
+    synth.calc_grid(M)
+    M.kbot[2:nx + 2, 2:ny + 2] = 1
+    M.kbot[2 + nx // 2:4 + nx // 2, 2 + ny // 2] = min(nz, 1 + nz // 2)  # a sill
+    M.kbot[2 + nx // 3, 2 + ny // 3] = 0 if ny > 1 else 1  # a column of land
+    synth.calc_topo(M)
+    forc = np.zeros(M.shape2d + (nz,), order="F")
+    inner = (slice(2, -2), slice(2, -2))
+    forc[inner] = rng.standard_normal((nx, ny, nz))
+    wet = M.maskT > 0
+    wet[:2] = wet[-2:] = False
+    wet[:, :2] = wet[:, -2:] = False
+    forc[wet] -= forc[wet].mean()
+    return M, forc
+
+
+# one block; slices over several blocks, their own neighbours across the seam, odd last pieces; blocks cut in
+# y as well, re-entrant both ways; columns of 8 and 12 levels a thread; too deep or too large for the cluster
+@pytest.mark.parametrize("nx,ny,nz,cyc_x,cyc_y", [
+    (9, 1, 5, False, False), (17, 1, 8, True, False), (64, 1, 24, True, False), (160, 1, 60, True, False),
+    (37, 1, 90, False, False), (4, 33, 20, False, True), (24, 17, 7, True, True), (33, 21, 11, False, True),
+    (40, 36, 9, False, False), (240, 1, 80, True, False), (48, 40, 24, True, False), (16, 1, 2000, False, False),
+    (70, 41, 22, True, True)])
+def test_cluster_solve(oracle_lib, nx, ny, nz, cyc_x, cyc_y):
+    M, forc = tank(nx, ny, nz, cyc_x, cyc_y)
+    O, nh = oracle_lib.Oracle3D(M), NonHydrostatic(M)
+    cf = O.make_coeff()
+    for it in (1, 4, 12):  # the iterate itself, before rounding has had time to grow
+        want = np.zeros(forc.shape, order="F")
+        ro = O.congrad(cf, forc, want, eps=0.0, max_it=it)
+        for variant in (0, 1):
+            nh.set_variant(variant)
+            got = np.zeros(forc.shape, order="F")
+            with warnings.catch_warnings():
+                warnings.simplefilter("ignore")
+                n, info = nh.congrad_non_hydro(forc, got, eps=0.0, max_it=it)
+            assert n == ro["iterations"] and info["status"] == ro["status"], (variant, it, n, ro)
+            assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want), (variant, it)
+    nh.close()
