@@ -329,19 +329,28 @@ __global__ void k_sf_columns(StepDev s, double* fpx, double* fpy) {
   const int i = (int)(q % (s.nx + 4)) - 1, j = (int)(q / (s.nx + 4)) - 1;
   const bool inner = i >= 1 && i <= s.nx && j >= 1 && j <= s.ny;
   const size_t qe = fidx(s.nx, i + 1, j), qn = fidx(s.nx, i, j + 1);
+  const size_t o0 = (size_t)(s.tau - 1) * n2 * s.nz + q;
+  double* __restrict__ du0 = s.du + o0;
+  double* __restrict__ dv0 = s.dv + o0;
+  const double* __restrict__ ph = s.p_hydro;
+  const double* __restrict__ mixu = s.du_mix + q;
+  const double* __restrict__ mixv = s.dv_mix + q;
+  const double* __restrict__ mU = s.maskU + q;
+  const double* __restrict__ mV = s.maskV + q;
   double ax = 0.0, ay = 0.0;
-  for (int k = 1; k <= s.nz; k++) {
-    const size_t d = q4(s, q, k, s.tau);
-    double du = s.du[d], dv = s.dv[d];
+#pragma unroll 4
+  for (int k = 0; k < s.nz; k++) {
+    const size_t m = k * n2;
+    double du = du0[m], dv = dv0[m];
     if (inner) {  // solve_streamfct.f90:32-37
-      du = du - (s.p_hydro[q3(s, qe, k)] - s.p_hydro[q3(s, q, k)]) / (s.dxu[i + 1] * s.cost[j + 1]) * s.maskU[q3(s, q, k)];
-      dv = dv - (s.p_hydro[q3(s, qn, k)] - s.p_hydro[q3(s, q, k)]) / s.dyu[j + 1] * s.maskV[q3(s, q, k)];
-      s.du[d] = du;
-      s.dv[d] = dv;
+      du = du - (ph[qe + m] - ph[q + m]) / (s.dxu[i + 1] * s.cost[j + 1]) * mU[m];
+      dv = dv - (ph[qn + m] - ph[q + m]) / s.dyu[j + 1] * mV[m];
+      du0[m] = du;
+      dv0[m] = dv;
     }
     // :40-43
-    ax = ax + (du + s.du_mix[q3(s, q, k)]) * s.maskU[q3(s, q, k)] * s.dzt[k - 1];
-    ay = ay + (dv + s.dv_mix[q3(s, q, k)]) * s.maskV[q3(s, q, k)] * s.dzt[k - 1];
+    ax = ax + (du + mixu[m]) * mU[m] * s.dzt[k];
+    ay = ay + (dv + mixv[m]) * mV[m] * s.dzt[k];
   }
   fpx[q] = ax * s.hur[q];  // :44
   fpy[q] = ay * s.hvr[q];
@@ -382,39 +391,59 @@ __global__ void k_sf_psi(StepDev s, const double* psin, int nisle, const double*
   ps1[q] = p;
 }
 
+// (The time levels of u and v are distinct, so no store touches a load; without
+// saying so every level waited for the one before: 61 us at 256x256x20.)
 __global__ void k_sf_velocity(StepDev s) {
   const size_t n2 = (size_t)(s.nx + 4) * (s.ny + 4);
   const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (q >= n2) return;
   const int i = (int)(q % (s.nx + 4)) - 1, j = (int)(q / (s.nx + 4)) - 1;
   const double AB = s.AB_eps, dt = s.dt_mom;
+  const size_t lev = n2 * s.nz, o0 = (size_t)(s.tau - 1) * lev + q, om = (size_t)(s.taum1 - 1) * lev + q;
+  double* __restrict__ u1 = s.u + (size_t)(s.taup1 - 1) * lev + q;
+  double* __restrict__ v1 = s.v + (size_t)(s.taup1 - 1) * lev + q;
+  const double* __restrict__ u0 = s.u + o0;
+  const double* __restrict__ v0 = s.v + o0;
+  const double* __restrict__ du0 = s.du + o0;
+  const double* __restrict__ dv0 = s.dv + o0;
+  const double* __restrict__ dum = s.du + om;
+  const double* __restrict__ dvm = s.dv + om;
+  const double* __restrict__ mixu = s.du_mix + q;
+  const double* __restrict__ mixv = s.dv_mix + q;
+  const double* __restrict__ mU = s.maskU + q;
+  const double* __restrict__ mV = s.maskV + q;
   double ax = 0.0, ay = 0.0;
-  for (int k = 1; k <= s.nz; k++) {  // :95-96 and :102-106
-    const size_t a1 = q4(s, q, k, s.taup1), a0 = q4(s, q, k, s.tau), am = q4(s, q, k, s.taum1), m = q3(s, q, k);
-    const double un = s.u[a0] + dt * (s.du_mix[m] + (1.5 + AB) * s.du[a0] - (0.5 + AB) * s.du[am]) * s.maskU[m];
-    const double vn = s.v[a0] + dt * (s.dv_mix[m] + (1.5 + AB) * s.dv[a0] - (0.5 + AB) * s.dv[am]) * s.maskV[m];
-    s.u[a1] = un;
-    s.v[a1] = vn;
-    ax = ax + un * s.maskU[m] * s.dzt[k - 1];
-    ay = ay + vn * s.maskV[m] * s.dzt[k - 1];
+#pragma unroll 4
+  for (int k = 0; k < s.nz; k++) {  // :95-96 and :102-106
+    const size_t m = k * n2;
+    const double un = u0[m] + dt * (mixu[m] + (1.5 + AB) * du0[m] - (0.5 + AB) * dum[m]) * mU[m];
+    const double vn = v0[m] + dt * (mixv[m] + (1.5 + AB) * dv0[m] - (0.5 + AB) * dvm[m]) * mV[m];
+    u1[m] = un;
+    v1[m] = vn;
+    ax = ax + un * mU[m] * s.dzt[k];
+    ay = ay + vn * mV[m] * s.dzt[k];
   }
   const bool inner = i >= 1 && i <= s.nx && j >= 1 && j <= s.ny;
   const double* ps1 = s.psi + (size_t)(s.taup1 - 1) * n2;
-  double gu = 0.0, gv = 0.0;
+  const double hur = s.hur[q], hvr = s.hvr[q];
+  double gu = 0.0, gv = 0.0, dy = 1.0, dx = 1.0;
   if (inner) {
     gu = ps1[q] - ps1[fidx(s.nx, i, j - 1)];
     gv = ps1[q] - ps1[fidx(s.nx, i - 1, j)];
+    dy = s.dyt[j + 1];
+    dx = s.cosu[j + 1] * s.dxt[i + 1];
   }
-  for (int k = 1; k <= s.nz; k++) {  // :107-118
-    const size_t a1 = q4(s, q, k, s.taup1), m = q3(s, q, k);
-    double un = s.u[a1] - ax * s.maskU[m] * s.hur[q];
-    double vn = s.v[a1] - ay * s.maskV[m] * s.hvr[q];
+#pragma unroll 4
+  for (int k = 0; k < s.nz; k++) {  // :107-118
+    const size_t m = k * n2;
+    double un = u1[m] - ax * mU[m] * hur;
+    double vn = v1[m] - ay * mV[m] * hvr;
     if (inner) {
-      un = un - s.maskU[m] * gu / s.dyt[j + 1] * s.hur[q];
-      vn = vn + s.maskV[m] * gv / (s.cosu[j + 1] * s.dxt[i + 1]) * s.hvr[q];
+      un = un - mU[m] * gu / dy * hur;
+      vn = vn + mV[m] * gv / dx * hvr;
     }
-    s.u[a1] = un;
-    s.v[a1] = vn;
+    u1[m] = un;
+    v1[m] = vn;
   }
 }
 

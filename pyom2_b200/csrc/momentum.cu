@@ -72,14 +72,18 @@ __device__ __forceinline__ double ipow(double x, int n) {
   return r;
 }
 
+constexpr int kCellThreads = 128;  // along i; the grid covers (i, j, k)
+
 // ---- Coriolis, metric terms, wind stress, advection -> du, dv(tau) ---------------
 // momentum.f90:11-35 (du_cor, dv_cor), :82-93 (du = du_cor, stress), :95-97 (+ du_adv);
 // momentum_advection.f90:13-76.
-__global__ void k_mom_cor_adv(MomDev m) {
+// One thread per cell: a thread per column left 14 warps on an SM at 256x256x20,
+// each waiting for its loads level by level (109 us).  The flux through the
+// bottom face is formed again from the cell below's expression.
+__global__ void __launch_bounds__(kCellThreads) k_mom_cor_adv(MomDev m) {
   const MG& g = m.g;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.nx * g.ny) return;
-  const int i = 1 + t % g.nx, j = 1 + t / g.nx;
+  const int i = 1 + blockIdx.x * kCellThreads + threadIdx.x, j = 1 + blockIdx.y;
+  if (i > g.nx) return;
   const int tau = m.tau, nz = g.nz;
   const double* ut = m.u + (size_t)(tau - 1) * g.n2 * nz;
   const double* vt = m.v + (size_t)(tau - 1) * g.n2 * nz;
@@ -98,8 +102,15 @@ __global__ void k_mom_cor_adv(MomDev m) {
   auto wtr = [&](int ii, int jj, int k) {
     return m.area_t[g.ij(ii, jj)] * wt[g.k3(ii, jj, k)] * m.maskW[g.k3(ii, jj, k)];
   };
-  double ftu_prev = 0.0, ftv_prev = 0.0;  // flux_top(k-1) of the u and v equations
-  for (int k = 1; k <= nz; k++) {
+  // flux_top of the u and v equations at level k
+  auto ftu = [&](int k) {
+    return k < nz ? 0.25 * (ut[g.k3(i, j, k + 1)] + ut[g.k3(i, j, k)]) * (wtr(i, j, k) + wtr(i + 1, j, k)) : 0.0;
+  };
+  auto ftv = [&](int k) {
+    return k < nz ? 0.25 * (vt[g.k3(i, j, k + 1)] + vt[g.k3(i, j, k)]) * (wtr(i, j, k) + wtr(i, j + 1, k)) : 0.0;
+  };
+  {
+    const int k = 1 + blockIdx.z;
     const size_t c = g.k3(i, j, k);
     const double mU = m.maskU[c], mV = m.maskV[c];
     // Coriolis (momentum.f90:13-16)
@@ -139,13 +150,11 @@ __global__ void k_mom_cor_adv(MomDev m) {
       const double fs =
           0.25 * (ut[g.k3(i, j - 1, k)] + ut[g.k3(i, j, k)]) * (vtr(i + 1, j - 1, k) + vtr(i, j - 1, k));
       double adv = -(mU * (fe - fw + fn - fs) / (area_u * m.dzt[k - 1]));
-      const double ft =
-          k < nz ? 0.25 * (ut[g.k3(i, j, k + 1)] + ut[g.k3(i, j, k)]) * (wtr(i, j, k) + wtr(i + 1, j, k)) : 0.0;
+      const double ft = ftu(k);
       if (k == 1)
         adv = adv - mU * ft / (area_u * m.dzt[k - 1]);
       else
-        adv = adv - mU * (ft - ftu_prev) / (area_u * m.dzt[k - 1]);
-      ftu_prev = ft;
+        adv = adv - mU * (ft - ftu(k - 1)) / (area_u * m.dzt[k - 1]);
       du_t = du_t + adv;
     }
     // advection of v (:46-69)
@@ -156,13 +165,11 @@ __global__ void k_mom_cor_adv(MomDev m) {
       const double fn = 0.25 * (vt[g.k3(i, j, k)] + vt[g.k3(i, j + 1, k)]) * (vtr(i, j + 1, k) + vtr(i, j, k));
       const double fs = 0.25 * (vt[g.k3(i, j - 1, k)] + vt[g.k3(i, j, k)]) * (vtr(i, j, k) + vtr(i, j - 1, k));
       double adv = -(mV * (fe - fw + fn - fs) / (area_v * m.dzt[k - 1]));
-      const double ft =
-          k < nz ? 0.25 * (vt[g.k3(i, j, k + 1)] + vt[g.k3(i, j, k)]) * (wtr(i, j, k) + wtr(i, j + 1, k)) : 0.0;
+      const double ft = ftv(k);
       if (k == 1)
         adv = adv - mV * ft / (area_v * m.dzt[k - 1]);
       else
-        adv = adv - mV * (ft - ftv_prev) / (area_v * m.dzt[k - 1]);
-      ftv_prev = ft;
+        adv = adv - mV * (ft - ftv(k - 1)) / (area_v * m.dzt[k - 1]);
       dv_t = dv_t + adv;
     }
     m.du[g.k4(i, j, k, tau)] = du_t;
@@ -177,68 +184,86 @@ __global__ void k_mom_cor_adv(MomDev m) {
 // reference's scratch), then du_mix = (u(taup1) - u(tau)) / dt_mom.
 constexpr int kMaxNz = 128;
 
-__global__ void k_mom_implicit(MomDev m, int uv) {
+// u and v in one launch (blockIdx.y); the loads of a level do not depend on the
+// recurrence, so they are issued a few levels ahead of it.
+__global__ void k_mom_implicit(MomDev m) {
   const MG& g = m.g;
+  const int uv = blockIdx.y;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.nx * g.ny) return;
   const int i = 1 + t % g.nx, j = 1 + t / g.nx;
   const int nz = g.nz;
   const int i1 = uv == 0 ? i + 1 : i, j1 = uv == 0 ? j : j + 1;  // the neighbour sharing the point
-  const double* mask = uv == 0 ? m.maskU : m.maskV;
+  const size_t n2 = g.n2, c0 = g.k3(i, j, 1), c1 = g.k3(i1, j1, 1);
+  const double* __restrict__ mask = (uv == 0 ? m.maskU : m.maskV) + c0;
+  const double* __restrict__ kap0 = m.kappaM + c0;
+  const double* __restrict__ kap1 = m.kappaM + c1;
   double* q = uv == 0 ? m.u : m.v;
-  double* q_mix = uv == 0 ? m.du_mix : m.dv_mix;
-  const double* qt = q + (size_t)(m.tau - 1) * g.n2 * nz;
-  double* qn = q + (size_t)(m.taup1 - 1) * g.n2 * nz;
+  double* __restrict__ mix = (uv == 0 ? m.du_mix : m.dv_mix) + c0;
+  const double* __restrict__ qt = q + (size_t)(m.tau - 1) * n2 * nz + c0;   // tau and taup1 differ, so the
+  double* __restrict__ qn = q + (size_t)(m.taup1 - 1) * n2 * nz + c0;       // two levels never overlap
   if (!m.implicit_vert) {
-    for (int k = 1; k <= nz; k++) q_mix[g.k3(i, j, k)] = 0.0;  // momentum.f90:115-117
+    for (int k = 0; k < nz; k++) mix[k * n2] = 0.0;  // momentum.f90:115-117
     return;
   }
   const int ks = max(m.kbot[g.ij(i, j)], m.kbot[g.ij(i1, j1)]);
+  int first = 1;  // lowest level the back substitution has not covered
   if (ks > 0 && ks < nz) {
-    double delta[kMaxNz], cp[kMaxNz], dp[kMaxNz];
-    for (int k = ks; k <= nz - 1; k++) {
-      const double fxa = 0.5 * (m.kappaM[g.k3(i, j, k)] + m.kappaM[g.k3(i1, j1, k)]);
-      delta[k - 1] = m.dt_mom / m.dzw[k - 1] * fxa * mask[g.k3(i, j, k + 1)] * mask[g.k3(i, j, k)];
-    }
-    delta[nz - 1] = 0.0;
-    // a, b, c of :128-141
-    auto a = [&](int k) { return k == ks ? 0.0 : -delta[k - 2] / m.dzt[k - 1]; };
-    auto b = [&](int k) {
-      if (k == nz) return 1 + delta[nz - 2] / m.dzt[nz - 1];
-      if (k == ks) return 1 + delta[k - 1] / m.dzt[k - 1];
-      return 1 + delta[k - 1] / m.dzt[k - 1] + delta[k - 2] / m.dzt[k - 1];
+    double cp[kMaxNz], dp[kMaxNz];
+    // delta(k) between levels k and k+1 (:118-125)
+    auto delta = [&](int k) {
+      const double fxa = 0.5 * (kap0[(k - 1) * n2] + kap1[(k - 1) * n2]);
+      return m.dt_mom / m.dzw[k - 1] * fxa * mask[k * n2] * mask[(k - 1) * n2];
     };
-    auto cc = [&](int k) { return k == nz ? 0.0 : -delta[k - 1] / m.dzt[k - 1]; };
-    cp[ks - 1] = cc(ks) / b(ks);
-    dp[ks - 1] = qt[g.k3(i, j, ks)] / b(ks);
-    for (int k = ks + 1; k <= nz; k++) {
-      const double mm = b(k) - cp[k - 2] * a(k);
-      const double fxa = 1.0 / mm;
-      cp[k - 1] = cc(k) * fxa;
-      dp[k - 1] = (qt[g.k3(i, j, k)] - dp[k - 2] * a(k)) * fxa;
+    // a, b, c of :128-141, with d = delta(k), dm = delta(k-1)
+    double d = delta(ks);
+    {
+      const double b = 1 + d / m.dzt[ks - 1];
+      cp[ks - 1] = -d / m.dzt[ks - 1] / b;
+      dp[ks - 1] = qt[(ks - 1) * n2] / b;
     }
-    double x = dp[nz - 1];
-    qn[g.k3(i, j, nz)] = x;
+    double cpm = cp[ks - 1], dpm = dp[ks - 1];
+#pragma unroll 4
+    for (int k = ks + 1; k <= nz; k++) {
+      const double dm = d;
+      d = k < nz ? delta(k) : 0.0;
+      const double dz = m.dzt[k - 1];
+      const double a = -dm / dz;
+      const double b = k == nz ? 1 + dm / dz : 1 + d / dz + dm / dz;
+      const double c = k == nz ? 0.0 : -d / dz;
+      const double mm = b - cpm * a;
+      const double fxa = 1.0 / mm;
+      cp[k - 1] = cpm = c * fxa;
+      dp[k - 1] = dpm = (qt[(k - 1) * n2] - dpm * a) * fxa;
+    }
+    double x = dpm;
+    qn[(nz - 1) * n2] = x;
+    mix[(nz - 1) * n2] = (x - qt[(nz - 1) * n2]) / m.dt_mom;
+#pragma unroll 4
     for (int k = nz - 1; k >= ks; k--) {
       x = dp[k - 1] - cp[k - 1] * x;
-      qn[g.k3(i, j, k)] = x;
+      qn[(k - 1) * n2] = x;
+      mix[(k - 1) * n2] = (x - qt[(k - 1) * n2]) / m.dt_mom;
     }
+    first = ks;
   } else if (ks == nz) {
     // one wet cell: the reference's b(nz) reads delta(nz-1) left over from an
     // earlier column (vertical_friction.f90:135); without coupling the cell
     // keeps its velocity here
-    qn[g.k3(i, j, nz)] = qt[g.k3(i, j, nz)];
+    qn[(nz - 1) * n2] = qt[(nz - 1) * n2];
+    first = nz + 1;
+  } else {
+    first = nz + 1;
   }
-  for (int k = 1; k <= nz; k++) q_mix[g.k3(i, j, k)] = (qn[g.k3(i, j, k)] - qt[g.k3(i, j, k)]) / m.dt_mom;
+  for (int k = 1; k < first; k++) mix[(k - 1) * n2] = (qn[(k - 1) * n2] - qt[(k - 1) * n2]) / m.dt_mom;
 }
 
 // ---- harmonic lateral friction and linear bottom friction -> du_mix, dv_mix ------
 // harmonic_friction.f90:11-39 (u) and :69-94 (v); bottom_friction.f90:110-135.
-__global__ void k_mom_lateral(MomDev m) {
+__global__ void __launch_bounds__(kCellThreads) k_mom_lateral(MomDev m) {
   const MG& g = m.g;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.nx * g.ny) return;
-  const int i = 1 + t % g.nx, j = 1 + t / g.nx;
+  const int i = 1 + blockIdx.x * kCellThreads + threadIdx.x, j = 1 + blockIdx.y;
+  if (i > g.nx) return;
   const int nz = g.nz, tau = m.tau;
   const double* ut = m.u + (size_t)(tau - 1) * g.n2 * nz;
   const double* vt = m.v + (size_t)(tau - 1) * g.n2 * nz;
@@ -270,7 +295,8 @@ __global__ void k_mom_lateral(MomDev m) {
   };
   const int kbu = max(m.kbot[g.ij(i, j)], m.kbot[g.ij(i + 1, j)]);
   const int kbv = max(m.kbot[g.ij(i, j + 1)], m.kbot[g.ij(i, j)]);
-  for (int k = 1; k <= nz; k++) {
+  {
+    const int k = 1 + blockIdx.z;
     const size_t c = g.k3(i, j, k);
     double dum = m.du_mix[c], dvm = m.dv_mix[c];
     if (m.hor_friction) {
@@ -333,12 +359,16 @@ __global__ void k_vertical_velocity(MomDev m, int lev) {
   double* wl = m.w + (size_t)(lev - 1) * g.n2 * g.nz;
   const double ct = m.cost[j + 1], dx = m.dxt[i + 1], dy = m.dyt[j + 1], cu = m.cosu[j + 1], cum = m.cosu[j];
   double prev = 0.0;
+  const double* __restrict__ u0 = ul;
+  const double* __restrict__ v0 = vl;
+  double* __restrict__ w0 = wl;
+#pragma unroll 4
   for (int k = 1; k <= g.nz; k++) {
-    const double div = (ul[g.k3(i, j, k)] - ul[g.k3(i - 1, j, k)]) / (ct * dx) +
-                       (cu * vl[g.k3(i, j, k)] - cum * vl[g.k3(i, j - 1, k)]) / (ct * dy);
+    const double div = (u0[g.k3(i, j, k)] - u0[g.k3(i - 1, j, k)]) / (ct * dx) +
+                       (cu * v0[g.k3(i, j, k)] - cum * v0[g.k3(i, j - 1, k)]) / (ct * dy);
     const double wk = k == 1 ? -m.maskW[g.k3(i, j, k)] * m.dzt[k - 1] * div
                              : prev - m.maskW[g.k3(i, j, k)] * m.dzt[k - 1] * div;
-    wl[g.k3(i, j, k)] = wk;
+    w0[g.k3(i, j, k)] = wk;
     prev = wk;
   }
 }
@@ -415,10 +445,10 @@ extern "C" int32_t pyomgpu_momentum_tendencies(pyomgpu_ctx* c, const pyomgpu_mom
   const MomDev m = to_dev(p, nx, ny, g1);
   cudaStream_t st = (cudaStream_t)stream;
   const int n = nx * ny, tb = 128, nb = (n + tb - 1) / tb;
-  k_mom_cor_adv<<<nb, tb, 0, st>>>(m);
-  k_mom_implicit<<<nb, tb, 0, st>>>(m, 0);
-  k_mom_implicit<<<nb, tb, 0, st>>>(m, 1);
-  k_mom_lateral<<<nb, tb, 0, st>>>(m);
+  const dim3 cells((nx + kCellThreads - 1) / kCellThreads, ny, m.g.nz);
+  k_mom_cor_adv<<<cells, kCellThreads, 0, st>>>(m);
+  k_mom_implicit<<<dim3(nb, 2), tb, 0, st>>>(m);
+  k_mom_lateral<<<cells, kCellThreads, 0, st>>>(m);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return mfail(PYOMGPU_ECUDA, "momentum kernels: %s", cudaGetErrorString(e));
   return PYOMGPU_OK;
