@@ -1220,16 +1220,31 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
     if (h->variant == 2) return nfail(PYOMGPU_ECUDA, "congrad_non_hydro: a cluster of %d blocks cannot be placed", C);
     // automatic choice: the brick kernel below
   }
-  // brick shape: 32 x ty x kc, ty the largest power of two <= min(8, ny), kc = (8/ty) kw with kw the
-  // largest level count per warp whose pipeline stages leave room for two blocks per SM
+  // brick shape: 32 x ty x kc, ty the largest power of two <= min(8, ny), kc = (8/ty) kw with up to the
+  // largest level count per warp kw whose pipeline stages leave room for two blocks per SM.  Of these kw the one
+  // whose busiest block has the least to do, a brick costing about its levels and two more: a short last round
+  // of bricks, or idle SMs, cost more than flatter bricks' wider halos.  us per iteration, kc = 7 and the choice:
+  // 60 x 60 x 20 10.86, 8.78 (3); 100 x 100 x 30 13.66, 13.07 (6); 120 x 120 x 40 18.31, 16.65 (5);
+  // 180 x 180 x 60 36.2, 35.5 (6); 240 x 240 x 80 keeps 7 (74.2; 77.6 with 5).  Fewer than 3 levels a warp lose
+  // to the march's start (60 x 60 x 20: 9.38 with 2).
   int ty = h->ty, kc = h->kc, ns = h->ns > 0 ? h->ns : 2;
   if (ty == 0) {
     ty = h->G.g.ny >= 8 ? 8 : h->G.g.ny >= 4 ? 4 : h->G.g.ny >= 2 ? 2 : 1;
     const int seg = 8 / ty;
-    const int kw_need = (h->G.nz + seg - 1) / seg;
-    int kw = 1;
-    while (kw < kw_need && nh_smem_bytes(ty, seg * (kw + 1), ns) <= (size_t)113 * 1024) kw++;
-    kc = seg * kw;
+    const int kw_need = (h->G.nz + seg - 1) / seg, nblk = h->grid > 0 ? std::min(h->grid, 2 * h->nsm) : 2 * h->nsm;
+    auto fits = [&](int kw) { return nh_smem_bytes(ty, seg * kw, ns) <= (size_t)113 * 1024; };
+    int kw0 = std::min(3, kw_need);
+    while (kw0 > 1 && !fits(kw0)) kw0--;
+    const long long cols = (long long)((h->G.g.nx + 31) / 32) * ((h->G.g.ny + ty - 1) / ty);
+    long long least = 0;
+    for (int kw = kw0; kw <= kw_need && (kw == kw0 || fits(kw)); kw++) {
+      const long long bricks = cols * ((h->G.nz + seg * kw - 1) / (seg * kw));
+      const long long cost = (bricks + nblk - 1) / nblk * (kw + 2);
+      if (kw == kw0 || cost < least) {
+        kc = seg * kw;
+        least = cost;
+      }
+    }
   }
   while (ns > 2 && nh_smem_bytes(ty, kc, ns) > kNHSmemMax) ns--;
   const size_t smem = nh_smem_bytes(ty, kc, ns);
