@@ -174,7 +174,8 @@ int32_t pyomgpu_set_sync_timeout(pyomgpu_ctx* ctx, double seconds);
 int32_t pyomgpu_inject_barrier_stall(pyomgpu_ctx* ctx, int32_t enable);
 
 /* CG kernel of the streamfunction solves (congrad_streamfunction,
- * solve_streamfunction, solve_rtol F64, the learned solver's fallback):
+ * solve_streamfunction, solve_rtol F64, the learned solver's fallback) and of
+ * the surface-pressure solves (congrad_surf_press, solve_pressure):
  * 1 = the tiled kernel (any grid; the one pyomgpu_autotune tunes),
  * 2 = the on-chip-resident kernel (one piece of the grid per SM, with the
  *     direction and face couplings in shared memory and the residual,
@@ -185,9 +186,11 @@ int32_t pyomgpu_inject_barrier_stall(pyomgpu_ctx* ctx, int32_t enable);
  *     recurrence and the reference's (p, Ap) by its exact bilinear expansion
  *     in products of the sweep before; the reference's stopping tests are
  *     evaluated one reduction later, on the same quantities),
- * 0 = automatic (2 wherever the grid fits: the reference's own recurrences;
- *     at 1440 x 720 3 runs on par with it).  PYOMGPU_EINVAL for 2 or 3 on a
- * grid that does not fit.  The surface-pressure solve always uses 1.
+ * 0 = automatic: small grids (up to about 48 000 points) in one thread-block
+ *     cluster, all fields in its shared memory and registers, else 2 wherever
+ *     the grid fits, else 1.  PYOMGPU_EINVAL for 2 or 3 on a grid that does
+ *     not fit.  The surface-pressure solve has no form of 3 (it runs 2) and
+ * runs 1 where the grid does not fit or maskT is not all zeros and ones.
  * Reduction order and recurrences differ between the kernels: results
  * change at rounding level. */
 int32_t pyomgpu_set_cg_kernel(pyomgpu_ctx* ctx, int32_t kernel);
@@ -473,10 +476,13 @@ int32_t pyomgpu_nh_set_brick(pyomgpu_nh* nh, int32_t ty, int32_t kc);
 /* TMA pipeline depth of the CG sweeps: 2..4 stages (0 = automatic, 2). */
 int32_t pyomgpu_nh_set_stages(pyomgpu_nh* nh, int32_t stages);
 /* CG kernel: 1 = the grid-wide brick kernel, 2 = one thread-block cluster
- * (up to 16 blocks) with the fields resident in distributed shared memory
- * (grids of at most 110704 cells; cluster barriers instead of grid barriers,
- * so the barrier-stall hook does not apply), 0 = automatic (2 up to 32768
- * cells).  Reduction order differs, results change at rounding level. */
+ * (up to 16 blocks) with the fields in registers and shared memory, where
+ * the grid can be cut into pieces of whole columns that fit (x-z slices up to
+ * about 27 000 cells, 3-D grids up to about 49 000), else one with them in
+ * distributed shared memory (grids of at most 110704 cells; cluster barriers,
+ * so the barrier-stall hook does not apply to it), 0 = automatic (the first
+ * where it fits, the second up to 32768 cells, else 1).  Reduction order
+ * differs, results change at rounding level. */
 int32_t pyomgpu_nh_set_variant(pyomgpu_nh* nh, int32_t variant);
 /* res = A p1 over the interior, zero halo (apply_op_3D).  (nx+4, ny+4, nz)
  * Fortran-layout arrays, host or device. */

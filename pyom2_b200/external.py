@@ -149,11 +149,13 @@ class ExternalMode:
         _abi.check(self._L.pyomgpu_inject_barrier_stall(self._ctx, int(bool(enable))))
 
     def set_cg_kernel(self, kernel: str = "auto"):
-        """CG kernel of the streamfunction solves: ``"tiled"`` (any grid),
+        """CG kernel of the solves: ``"tiled"`` (any grid),
         ``"resident"`` (one piece of the grid per SM, held on chip for the
         whole solve, two reductions per iteration as the reference),
         ``"resident1"`` (the same with one reduction per iteration) or
-        ``"auto"``; the resident ones raise on a grid that does not fit."""
+        ``"auto"`` (small grids in one thread-block cluster, else resident
+        where the grid fits, else tiled); the resident ones raise on a grid
+        that does not fit (surface-pressure solves run tiled there)."""
         code = {"auto": 0, "tiled": 1, "resident": 2, "resident1": 3}[kernel]
         _abi.check(self._L.pyomgpu_set_cg_kernel(self._ctx, code))
         self._cg_kernel = kernel

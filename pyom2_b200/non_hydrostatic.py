@@ -86,8 +86,8 @@ class NonHydrostatic:
         _abi.check(self._L.pyomgpu_nh_set_stages(self._h, int(stages)))
 
     def set_variant(self, variant: int):
-        """CG kernel: 1 grid-wide bricks, 2 one block resident in shared memory
-        (small grids), 0 automatic."""
+        """CG kernel: 1 grid-wide bricks, 2 one thread-block cluster with the
+        fields on chip (small grids), 0 automatic."""
         _abi.check(self._L.pyomgpu_nh_set_variant(self._h, int(variant)))
 
     def apply_op_3d(self, p):
