@@ -344,21 +344,28 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------- weights
-__global__ void k_pack_weights(const float* __restrict__ w, int cout, int cin, int flip, uint16_t* __restrict__ out) {
+// All packings of a network in one launch (blockIdx.y).  A launch for each took
+// 24 of them in a training step, 40 us of kernels and the gaps between them:
+// 1.50 ms at 1440 x 720, now 1.39.
+struct PackJobs {
+  WeightPack p[kMaxWeightPacks];
+};
+__global__ void k_pack_weights(const __grid_constant__ PackJobs jobs) {
   // out[dx][ci/8][2-dy][co][ci%8] = w[co][ci][3 dy + dx]; flip: input channels = forward cout, taps rotated
   // (dx -> 2-dx, dy -> 2-dy).  The three dy of a dx are neighbours in N, in the order of the output rows they
   // feed.
-  const int n = 9 * cin * cout;
+  const WeightPack& p = jobs.p[blockIdx.y];
+  const int cout = p.cout, cin = p.cin, n = 9 * cin * cout;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int co = e / (cin * 9), rem = e - co * cin * 9, ci = rem / 9, tap = rem - ci * 9;
     const int dy = tap / 3, dx = tap - 3 * dy;
-    const float v = w[e];
+    const float v = p.w[e];
     size_t o;
-    if (!flip)
+    if (!p.flip)
       o = (((size_t)(dx * (cin / 8) + ci / 8) * 3 + (2 - dy)) * cout + co) * 8 + (ci & 7);
     else
       o = (((size_t)((2 - dx) * (cout / 8) + co / 8) * 3 + dy) * cin + ci) * 8 + (co & 7);
-    out[o] = f2bf(v);
+    p.out[o] = f2bf(v);
   }
 }
 
@@ -445,9 +452,17 @@ int conv3x3_launch(const ConvSpec& s, int nsm, cudaStream_t st) {
   return -1;
 }
 
-void launch_pack_weights(const float* w, int cout, int cin, bool flip, uint16_t* wpack, cudaStream_t st) {
-  const int n = 9 * cin * cout;
-  k_pack_weights<<<(n + 255) / 256, 256, 0, st>>>(w, cout, cin, flip ? 1 : 0, wpack);
+void launch_pack_weights(const WeightPack* packs, int count, cudaStream_t st) {
+  for (int k = 0; k < count; k += kMaxWeightPacks) {
+    PackJobs jobs{};
+    const int m = std::min(kMaxWeightPacks, count - k);
+    int most = 0;
+    for (int l = 0; l < m; l++) {
+      jobs.p[l] = packs[k + l];
+      most = std::max(most, 9 * packs[k + l].cin * packs[k + l].cout);
+    }
+    k_pack_weights<<<dim3((most + 255) / 256, m), 256, 0, st>>>(jobs);
+  }
 }
 
 }  // namespace pyomgpu

@@ -73,6 +73,13 @@ int conv3x3_dw_launch(int cin, int cout, const uint16_t* X, const uint16_t* G, i
 // to nearest even).  flip packs the backward-data kernel instead: channels
 // transposed and taps rotated by 180 degrees (its input channels are the
 // forward Cout).
-void launch_pack_weights(const float* w, int cout, int cin, bool flip, uint16_t* wpack, cudaStream_t st);
+struct WeightPack {
+  const float* w;
+  uint16_t* out;
+  int cout, cin;  // of w
+  bool flip;
+};
+constexpr int kMaxWeightPacks = 24;  // in one launch
+void launch_pack_weights(const WeightPack* packs, int count, cudaStream_t st);
 
 }  // namespace pyomgpu

@@ -60,10 +60,8 @@ int32_t pyomgpu_conv3x3_bf16(int32_t cin, int32_t cout, int32_t H, int32_t W, co
     return lfail(PYOMGPU_ENOMEM, "conv3x3: cudaMalloc");
   }
   // flip: w is the forward weight [cin][cout][3][3] of the layer this call differentiates
-  if (flip)
-    launch_pack_weights(w, cin, cout, true, wpack, st);
-  else
-    launch_pack_weights(w, cout, cin, false, wpack, st);
+  const WeightPack pack{w, wpack, flip ? cin : cout, flip ? cout : cin, flip != 0};
+  launch_pack_weights(&pack, 1, st);
   cudaMemsetAsync(err, 0, sizeof(int), st);
   ConvSpec s{};
   s.cin = cin;

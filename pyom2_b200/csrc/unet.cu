@@ -186,11 +186,14 @@ void unet_free(UNet& n) {
 }
 
 void unet_pack(UNet& n, cudaStream_t st) {
+  WeightPack packs[2 * kUNetLayers];
+  int m = 0;
   for (int l = 0; l < kUNetLayers; l++) {
     const float* w = n.params + unet_weight_offset(l);
-    launch_pack_weights(w, kUNet[l].cout, kUNet[l].cin, false, n.wpack[l], st);
-    if (n.training) launch_pack_weights(w, kUNet[l].cout, kUNet[l].cin, true, n.wflip[l], st);
+    packs[m++] = WeightPack{w, n.wpack[l], kUNet[l].cout, kUNet[l].cin, false};
+    if (n.training) packs[m++] = WeightPack{w, n.wflip[l], kUNet[l].cout, kUNet[l].cin, true};
   }
+  launch_pack_weights(packs, m, st);
 }
 
 namespace {
