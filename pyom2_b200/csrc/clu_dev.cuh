@@ -19,8 +19,10 @@ __device__ __forceinline__ uint32_t clu_map(uint32_t a, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
   return r;
 }
+// Not the .aligned form: that one is only defined where the whole warp executes it together, and the kernels come
+// here from stores that only some lanes make and out of waits that ran out.
 __device__ __forceinline__ void clu_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // two tagged words into a block of the cluster, and two of this block's; each
 // word is validated on its own, so the pair need not be single-copy atomic
