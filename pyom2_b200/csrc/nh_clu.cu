@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(NT, 1) nh_clu_kernel(const __grid_constant__ N
     for (int e = tid; e < nent * 4 + 8 * kCluMaxSlots * 2; e += NT) b[e] = 0ull;
     if (tid < 2) s_dead[tid] = 0;
   }
+  __syncthreads();  // the initial residual's loop reads the vertical factors of other warps
   const int rW = px > 0 ? rank - 1 : (CX ? rank + npx - 1 : -1), rE = px < npx - 1 ? rank + 1 : (CX ? rank - (npx - 1) : -1);
   const int rS = py > 0 ? rank - npx : (CY ? rank + npx * (npy - 1) : -1);
   const int rN = py < npy - 1 ? rank + npx : (CY ? rank - npx * (npy - 1) : -1);

@@ -57,3 +57,23 @@ def test_cluster_solve(oracle_lib, nx, ny, nz, cyc_x, cyc_y):
             assert n == ro["iterations"] and info["status"] == ro["status"], (variant, it, n, ro)
             assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want), (variant, it)
     nh.close()
+
+
+# a level's vertical factors are put into shared memory by one warp and read by others: segments of 4, 8 and 12
+# levels, columns of more levels than a warp has lanes, one block and several
+@pytest.mark.parametrize("nx,ny,nz", [(4, 1, 97), (16, 1, 300), (37, 1, 90), (20, 2, 70), (240, 1, 80), (24, 24, 67)])
+def test_deep_columns_repeat_to_the_bit(oracle_lib, nx, ny, nz):
+    M, forc = tank(nx, ny, nz, False, False)
+    O, nh = oracle_lib.Oracle3D(M), NonHydrostatic(M)
+    want = np.zeros(forc.shape, order="F")
+    O.congrad(O.make_coeff(), forc, want, eps=0.0, max_it=5)
+    first = None
+    for _ in range(20):
+        got = np.zeros(forc.shape, order="F")
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")
+            nh.congrad_non_hydro(forc, got, eps=0.0, max_it=5)
+        assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want)
+        first = got if first is None else first
+        assert np.array_equal(got, first)
+    nh.close()
