@@ -1169,7 +1169,11 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
   h->stall_next = 0;
   P.out = h->d_result;
   const size_t ncell = (size_t)h->G.g.nx * h->G.g.ny * h->G.nz;
-  if (h->variant != 1 && nh_clu_plan(h)) {
+  // a caller that sets the bricks' grid, shape or stages wants bricks; up to kNHClusterAuto cells the automatic
+  // choice is a cluster all the same, as those settings never chose the kernel there
+  const bool bricks_asked =
+      h->variant == 0 && ncell > (size_t)kNHClusterAuto && (h->grid > 0 || h->ty > 0 || h->ns > 0);
+  if (h->variant != 1 && !bricks_asked && nh_clu_plan(h)) {
     const NHCut& c = h->cut;
     P.cnpx = c.npx;
     P.cnpy = c.npy;

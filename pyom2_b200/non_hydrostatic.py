@@ -87,7 +87,8 @@ class NonHydrostatic:
 
     def set_variant(self, variant: int):
         """CG kernel: 1 grid-wide bricks, 2 one thread-block cluster with the
-        fields on chip (small grids), 0 automatic."""
+        fields on chip (small grids), 0 automatic (above 32768 cells bricks
+        wherever ``set_grid``, ``set_brick`` or ``set_stages`` is set)."""
         _abi.check(self._L.pyomgpu_nh_set_variant(self._h, int(variant)))
 
     def apply_op_3d(self, p):

@@ -77,3 +77,21 @@ def test_deep_columns_repeat_to_the_bit(oracle_lib, nx, ny, nz):
         first = got if first is None else first
         assert np.array_equal(got, first)
     nh.close()
+
+
+# 33 600 cells: the cluster kernel's by size, but a brick setting is for the bricks
+@pytest.mark.parametrize("call", [("set_grid", 7), ("set_brick", 4, 6), ("set_stages", 3)])
+def test_brick_settings_choose_the_bricks(call):
+    M, forc = tank(40, 40, 21, True, False)
+    out = []
+    for variant in (0, 1):
+        nh = NonHydrostatic(M)
+        nh.set_variant(variant)
+        getattr(nh, call[0])(*call[1:])
+        p = np.zeros(forc.shape, order="F")
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")
+            nh.congrad_non_hydro(forc, p, eps=0.0, max_it=20)
+        out.append(p)
+        nh.close()
+    assert np.array_equal(*out)
