@@ -96,3 +96,41 @@ def test_ensemble_with_momentum_physics_matches_the_host_path():
     assert np.abs(M.u).max() > 0
     ens.close()
     E.close()
+
+
+def _rows_of_period_16(nx, ny, nz):
+    """A plane channel of ny rows in which every field repeats after 16 rows."""
+    from pyom2_b200 import synth
+    from pyom2_b200.model import ModelState
+    M = ModelState(nx, ny, nz, enable_cyclic_x=True, coord_degree=False)
+    M.dxt[2:nx + 2], M.dyt[2:ny + 2], M.dzt[:] = 2e4, 2.5e4, 200.0
+    synth.calc_grid(M)
+    M.kbot[2:nx + 2, 2:ny + 2] = 1
+    synth.calc_topo(M)
+    rng = np.random.default_rng(5)
+    rows = np.arange(ny + 4) % 16
+    for n, size in (("u", 0.1), ("v", 0.1), ("w", 1e-4)):
+        getattr(M, n)[..., M.tau - 1] = size * rng.standard_normal((nx + 4, 16, nz))[:, rows]
+    M.kappaM[...] = 1e-3 * (1.0 + 0.5 * rng.uniform(size=(nx + 4, 16, nz)))[:, rows]
+    M.coriolis_t[...] = 1e-4
+    M.dt_mom, M.A_h, M.r_bot = 1800.0, 1e3, 1e-5
+    M.enable_hor_friction = M.enable_bottom_friction = M.enable_implicit_vert_friction = True
+    return M
+
+
+@pytest.mark.parametrize("nx,ny", [(4, 65600), (131, 80)])
+def test_every_row_of_a_long_channel(nx, ny):
+    """More rows than a launch has blocks in y, and a width just above a block's threads:
+    away from the walls each row equals the row it repeats, bit for bit."""
+    small, M = _rows_of_period_16(nx, 64, 3), _rows_of_period_16(nx, ny, 3)
+    for S in (small, M):
+        E = ExternalMode(S)
+        E.momentum(S)
+        E.close()
+    j = np.arange(24, ny - 24)
+    same = 24 + (j - 24) % 16
+    for n in MOMENTUM_OUT_3D:
+        a, b = getattr(M, n), getattr(small, n)
+        a, b = (x[:, :, :, M.tau - 1] if x.ndim == 4 else x for x in (a, b))
+        assert np.abs(b).max() > 0
+        assert np.array_equal(a[2:-2][:, j], b[2:-2][:, same]), n
