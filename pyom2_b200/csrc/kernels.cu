@@ -391,8 +391,11 @@ __global__ void k_sf_psi(StepDev s, const double* psin, int nisle, const double*
   ps1[q] = p;
 }
 
-// (The time levels of u and v are distinct, so no store touches a load; without
-// saying so every level waited for the one before: 61 us at 256x256x20.)
+// kInPlace: taup1 is tau.  Where they are distinct no store touches a load;
+// without saying so every level waited for the one before (60 us at
+// 256x256x20, 52 this way), also with four levels' loads ahead of their stores
+// (62).
+template <bool kInPlace>
 __global__ void k_sf_velocity(StepDev s) {
   const size_t n2 = (size_t)(s.nx + 4) * (s.ny + 4);
   const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -416,8 +419,9 @@ __global__ void k_sf_velocity(StepDev s) {
 #pragma unroll 4
   for (int k = 0; k < s.nz; k++) {  // :95-96 and :102-106
     const size_t m = k * n2;
-    const double un = u0[m] + dt * (mixu[m] + (1.5 + AB) * du0[m] - (0.5 + AB) * dum[m]) * mU[m];
-    const double vn = v0[m] + dt * (mixv[m] + (1.5 + AB) * dv0[m] - (0.5 + AB) * dvm[m]) * mV[m];
+    const double uo = kInPlace ? u1[m] : u0[m], vo = kInPlace ? v1[m] : v0[m];
+    const double un = uo + dt * (mixu[m] + (1.5 + AB) * du0[m] - (0.5 + AB) * dum[m]) * mU[m];
+    const double vn = vo + dt * (mixv[m] + (1.5 + AB) * dv0[m] - (0.5 + AB) * dvm[m]) * mV[m];
     u1[m] = un;
     v1[m] = vn;
     ax = ax + un * mU[m] * s.dzt[k];
@@ -713,7 +717,10 @@ void launch_sf_psi_update(const StepDev& s, const double* psin, int nisle, const
 
 void launch_sf_velocity_update(const StepDev& s, cudaStream_t st) {
   const size_t n2 = (size_t)(s.nx + 4) * (s.ny + 4);
-  k_sf_velocity<<<nblk(n2, 128), 128, 0, st>>>(s);
+  if (s.taup1 == s.tau)
+    k_sf_velocity<true><<<nblk(n2, 128), 128, 0, st>>>(s);
+  else
+    k_sf_velocity<false><<<nblk(n2, 128), 128, 0, st>>>(s);
 }
 
 void launch_sp_forcing(const StepDev& s, int free_surface, double* fpx, double* fpy, double* forc, cudaStream_t st) {

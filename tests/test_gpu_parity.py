@@ -297,3 +297,28 @@ def test_status_nan_maxiter_timeout(oracle_lib):
     s = np.zeros(Mg.shape2d, order="F")
     it, conv, _ = E.congrad_streamfunction(W.forc, s)  # the context is still usable
     assert conv and it > 10
+
+
+@pytest.mark.parametrize("nz", [1, 3, 4, 6])
+def test_solve_streamfunction_step_in_place(nz):
+    """taup1 may be tau: the step then updates u, v and psi where they are.  With AB_eps = -1/2 only the
+    tendencies at tau count and the old dpsi drops out, so every value is that of a step into another level."""
+    import warnings
+
+    W = synth.config4(77, nx=48, ny=32, nz=nz)
+    Mi = W.M
+    random_state(Mi, 6)
+    Mi.AB_eps = -0.5
+    Mo = Mi.copy()
+    Mi.taup1 = Mi.tau
+    for M in (Mi, Mo):
+        E = ExternalMode(M)
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore", RuntimeWarning)
+            E.streamfunction_init()
+            E.solve_streamfunction(M)
+        E.close()
+    assert Mi.congr_itts == Mo.congr_itts > 0
+    for n in ("dpsi", "psi", "u", "v"):
+        a, b = getattr(Mi, n)[..., Mi.taup1 - 1], getattr(Mo, n)[..., Mo.taup1 - 1]
+        assert np.array_equal(a, b), n
