@@ -195,8 +195,15 @@ int32_t pyomgpu_inject_barrier_stall(pyomgpu_ctx* ctx, int32_t enable);
  * change at rounding level. */
 int32_t pyomgpu_set_cg_kernel(pyomgpu_ctx* ctx, int32_t kernel);
 /* Piece layout the resident kernel uses on this grid: pieces in x and y and
- * points per thread; PYOMGPU_EINVAL when the grid does not fit. */
+ * points per thread; PYOMGPU_EINVAL when the grid does not fit.  (Where the
+ * automatic choice takes a cluster, only 2, 3 and traced solves use it.) */
 int32_t pyomgpu_resident_layout(pyomgpu_ctx* ctx, int32_t* npx, int32_t* npy, int32_t* points_per_thread);
+/* Cut of this grid in the one-cluster kernel (fp32: of its FP32 form, for the
+ * correction solves of pyomgpu_solve_rtol with PYOMGPU_PREC_F32): pieces in x
+ * and y (their product is the cluster's blocks), threads per block and points
+ * per thread; PYOMGPU_EINVAL where the automatic choice takes another kernel. */
+int32_t pyomgpu_cluster_layout(pyomgpu_ctx* ctx, int32_t fp32, int32_t* npx, int32_t* npy, int32_t* threads,
+                               int32_t* points_per_thread);
 /* The same for the FP32 resident kernel that runs the correction solves of
  * pyomgpu_solve_rtol with PYOMGPU_PREC_F32 where the grid fits (FP32 fields
  * take half the on-chip memory, so grids up to twice the size fit; elsewhere,

@@ -1772,6 +1772,19 @@ int32_t pyomgpu_resident_layout32(pyomgpu_ctx* c, int32_t* npx, int32_t* npy, in
   return PYOMGPU_OK;
 }
 
+int32_t pyomgpu_cluster_layout(pyomgpu_ctx* c, int32_t fp32, int32_t* npx, int32_t* npy, int32_t* threads,
+                               int32_t* points_per_thread) {
+  if (!c || (fp32 != 0 && fp32 != 1)) return fail(PYOMGPU_EINVAL, "cluster layout: bad arguments");
+  if (int rc = clu_plan(c, fp32 != 0)) return rc;
+  const ResCut& cut = c->resd.clu[fp32];
+  if (cut.npx == 0) return fail(PYOMGPU_EINVAL, "the automatic choice runs no cluster on this grid");
+  if (npx) *npx = cut.npx;
+  if (npy) *npy = cut.npy;
+  if (threads) *threads = cut.nt;
+  if (points_per_thread) *points_per_thread = cut.p;
+  return PYOMGPU_OK;
+}
+
 int32_t pyomgpu_set_psin_solve(pyomgpu_ctx* c, double rtol, int32_t weighted) {
   if (!c || rtol < 0.0 || rtol >= 1.0 || (weighted != 0 && weighted != 1))
     return fail(PYOMGPU_EINVAL, "set_psin_solve: bad arguments");

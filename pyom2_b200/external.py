@@ -161,12 +161,27 @@ class ExternalMode:
         self._cg_kernel = kernel
 
     def resident_kernel_name(self):
-        """Name of the resident kernel instance the current choice launches."""
+        """Name of the on-chip kernel instance the current choice launches."""
+        if getattr(self, "_cg_kernel", "auto") == "auto":
+            clu = self.cluster_layout()
+            if clu is not None:
+                return f"cg_clu_kernel<{clu[2]},{clu[3]}>"
         lay = self.resident_layout()
         if lay is None:
             return None
         single = getattr(self, "_cg_kernel", "auto") == "resident1"
         return f"cg_res{'1' if single else ''}_kernel<{lay[2]}>"
+
+    def cluster_layout(self, fp32: bool = False):
+        """(pieces in x, pieces in y, threads per block, points per thread)
+        of the one-cluster kernel on this grid (``fp32``: of its FP32 form),
+        or None where the automatic choice takes another kernel."""
+        v = [C.c_int32() for _ in range(4)]
+        rc = self._L.pyomgpu_cluster_layout(self._ctx, int(bool(fp32)), *(C.byref(x) for x in v))
+        if rc == _abi.EINVAL:
+            return None
+        _abi.check(rc)
+        return tuple(x.value for x in v)
 
     def resident_layout(self, fp32: bool = False):
         """(pieces in x, pieces in y, points per thread) of the resident

@@ -72,3 +72,25 @@ def test_cluster_solve_to_residual(nx, ny, precision):
         assert info["status"] == 0 and info["rel_residual"] <= 1e-11
         out[kernel] = x
     assert np.linalg.norm(out["auto"] - out["tiled"]) <= 1e-8 * np.linalg.norm(out["tiled"])
+
+
+@pytest.mark.parametrize("nx,ny", [(24, 20), (97, 83), (451, 387)])
+def test_the_layout_calls_name_the_kernel_that_runs(nx, ny):
+    from torch.profiler import ProfilerActivity, profile
+    M, forc = model(nx, ny, False, False)
+    E = ExternalMode(M)
+    for kernel in ("auto", "resident"):
+        E.set_cg_kernel(kernel)
+        name, args = E.resident_kernel_name()[:-1].split("<")
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            E.solve_rtol(forc, np.zeros(M.shape2d, order="F"), rtol=1e-3)
+        ran = [e.key for e in p.key_averages() if "cg_" in e.key]
+        assert len(ran) == 1 and f"{name}<" in ran[0], (name, ran)
+        if name == "cg_clu_kernel":
+            assert kernel == "auto" and f"<double, {args.replace(',', ', ')}, false>" in ran[0], (args, ran)
+        else:
+            assert name == "cg_res_kernel" and f"<{args}, " in ran[0], (args, ran)
+    npx_npy_nt_p = E.cluster_layout()
+    assert (npx_npy_nt_p is None) == (nx * ny > 48000) == (E.cluster_layout(fp32=True) is None)
+    if npx_npy_nt_p:
+        assert npx_npy_nt_p[0] * npx_npy_nt_p[1] <= 16
