@@ -95,3 +95,27 @@ def test_brick_settings_choose_the_bricks(call):
         out.append(p)
         nh.close()
     assert np.array_equal(*out)
+
+
+# grids that one cluster of whole columns does not hold: the compact cluster kernel, chosen automatically for deep
+# slices and by name up to 110704 cells, with neighbours and halo copies across the seams
+@pytest.mark.parametrize("nx,ny,nz,cyc_x,cyc_y,variant", [
+    (64, 1, 500, True, False, 0), (5, 5, 1300, True, True, 0), (97, 33, 17, True, False, 2),
+    (61, 47, 20, True, True, 2), (40, 60, 30, False, True, 2), (75, 41, 19, False, False, 2)])
+def test_compact_cluster_kernel(oracle_lib, nx, ny, nz, cyc_x, cyc_y, variant):
+    from torch.profiler import ProfilerActivity, profile
+    M, forc = tank(nx, ny, nz, cyc_x, cyc_y)
+    O, nh = oracle_lib.Oracle3D(M), NonHydrostatic(M)
+    nh.set_variant(variant)
+    cf = O.make_coeff()
+    start = np.asfortranarray(1e-3 * np.random.default_rng(nx).standard_normal(forc.shape))  # halo unlike the interior
+    for it in (1, 4, 12):
+        want, got = start.copy(order="F"), start.copy(order="F")
+        ro = O.congrad(cf, forc, want, eps=0.0, max_it=it)
+        with warnings.catch_warnings(), profile(activities=[ProfilerActivity.CUDA]) as p:
+            warnings.simplefilter("ignore")
+            n, info = nh.congrad_non_hydro(forc, got, eps=0.0, max_it=it)
+        assert any("nh_cg_small_kernel" in e.key for e in p.key_averages())
+        assert n == ro["iterations"] and info["status"] == ro["status"], (it, n, ro)
+        assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want), it
+    nh.close()
