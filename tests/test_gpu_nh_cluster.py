@@ -6,7 +6,7 @@ import warnings
 import numpy as np
 import pytest
 
-from pyom2_b200 import synth
+from pyom2_b200 import _abi, synth
 from pyom2_b200.model import ModelState
 from pyom2_b200.non_hydrostatic import NonHydrostatic
 
@@ -118,4 +118,47 @@ def test_compact_cluster_kernel(oracle_lib, nx, ny, nz, cyc_x, cyc_y, variant):
         assert any("nh_cg_small_kernel" in e.key for e in p.key_averages())
         assert n == ro["iterations"] and info["status"] == ro["status"], (it, n, ro)
         assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want), it
+    nh.close()
+
+
+# one block, several along x, a cut in x and y
+CUTS = [(9, 1, 5, False, False), (160, 1, 60, True, False), (24, 17, 7, True, True)]
+
+
+@pytest.mark.parametrize("nx,ny,nz,cyc_x,cyc_y", CUTS)
+def test_timeout_leaves_the_handle_usable(nx, ny, nz, cyc_x, cyc_y):
+    M, forc = tank(nx, ny, nz, cyc_x, cyc_y)
+    nh = NonHydrostatic(M)
+    want, got = (np.zeros(forc.shape, order="F") for _ in range(2))
+    n, info = nh.congrad_non_hydro(forc, want, eps=1e-9, max_it=5000)
+    assert info["status"] == _abi.OK and n > 3
+    nh.set_sync_timeout(0.2)
+    nh.inject_barrier_stall(True)
+    with pytest.raises(_abi.PyOMGPUError) as e:
+        nh.congrad_non_hydro(forc, np.zeros(forc.shape, order="F"), eps=1e-9)
+    assert e.value.code == _abi.TIMEOUT
+    again, info = nh.congrad_non_hydro(forc, got, eps=1e-9, max_it=5000)
+    assert info["status"] == _abi.OK and again == n and np.array_equal(got, want)
+    nh.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz,cyc_x,cyc_y", CUTS)
+def test_a_nan_ends_the_solve_and_the_halo_keeps_its_offset(oracle_lib, nx, ny, nz, cyc_x, cyc_y):
+    M, forc = tank(nx, ny, nz, cyc_x, cyc_y)
+    O, nh = oracle_lib.Oracle3D(M), NonHydrostatic(M)
+    start = np.asfortranarray(1e-3 * np.random.default_rng(3).standard_normal(forc.shape))
+    want, got = start.copy(order="F"), start.copy(order="F")
+    ro = O.congrad(O.make_coeff(), forc, want, eps=0.0, max_it=6)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        n, info = nh.congrad_non_hydro(forc, got, eps=0.0, max_it=6)
+    assert n == ro["iterations"] and np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want)
+    bad = forc.copy(order="F")
+    i, j, k = np.argwhere(M.maskT[2:-2, 2:-2] > 0)[5]
+    bad[i + 2, j + 2, k] = np.nan
+    for variant in (1, 0):
+        nh.set_variant(variant)
+        with pytest.raises(_abi.PyOMGPUError) as e:
+            nh.congrad_non_hydro(bad, np.zeros(forc.shape, order="F"), eps=1e-9)
+        assert e.value.code == _abi.NAN, variant
     nh.close()
