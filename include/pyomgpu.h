@@ -487,10 +487,11 @@ int32_t pyomgpu_nh_set_stages(pyomgpu_nh* nh, int32_t stages);
  * the grid can be cut into pieces of whole columns that fit (x-z slices up to
  * about 27 000 cells, 3-D grids up to about 49 000), else one with them in
  * distributed shared memory (grids of at most 110704 cells; cluster barriers,
- * so the barrier-stall hook does not apply to it), 0 = automatic (the first
- * where it fits, the second up to 32768 cells, else 1; above 32768 cells also
- * 1 where nh_set_grid, nh_set_brick or nh_set_stages is set).  Reduction
- * order differs, results change at rounding level. */
+ * so the barrier-stall hook does not apply to it) and on deep narrow grids,
+ * where that is faster, 0 = automatic (as 2 up to 32768 cells; above, the
+ * first where it fits and is faster than 1, unless nh_set_grid, nh_set_brick
+ * or nh_set_stages is set, else 1).  Reduction order differs, results change
+ * at rounding level. */
 int32_t pyomgpu_nh_set_variant(pyomgpu_nh* nh, int32_t variant);
 /* res = A p1 over the interior, zero halo (apply_op_3D).  (nx+4, ny+4, nz)
  * Fortran-layout arrays, host or device. */

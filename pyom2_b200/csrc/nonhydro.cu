@@ -1123,7 +1123,7 @@ bool nh_clu_plan(pyomgpu_nh* h) {
         const double c = nh_clu_iter_ns(h, npx, npy, w, hh, p, nt);
         if (c < cost) {
           cost = c;
-          best = NHCut{npx, npy, w, hh, p, nt, smem};
+          best = NHCut{npx, npy, w, hh, p, nt, smem, c};
         }
       }
     }
@@ -1141,6 +1141,27 @@ bool nh_clu_plan(pyomgpu_nh* h) {
     return false;
   }
   return true;
+}
+
+// Whether the cluster kernel is faster on its cut than what runs otherwise: the compact cluster kernel (up to
+// kNHClusterAuto cells, or asked for), or the bricks.  It exchanges whole faces through its blocks' inboxes, so on
+// deep narrow tanks, whose faces are large for their cells, it is not.  us per iteration, cluster and otherwise:
+// 6 x 6 x 400 11.56, 7.68; 4 x 4 x 600 9.59, 6.99; 8 x 8 x 400 14.73, 10.06; 16 x 16 x 170 14.12, 8.81 (bricks);
+// 20 x 20 x 110 12.89, 8.66 (bricks); but 8 x 8 x 100 4.59, 7.28; 16 x 16 x 120 8.89, 10.86; 60 x 60 x 12 7.38,
+// 8.56 (bricks).  The compact kernel makes one pass over its cells up to 16384, two or three above, and its halo
+// copies cost a cyclic grid more; the bricks of all grids this small are one a block, 8.4 to 9.6.  Over 166 grids the
+// rule takes the faster one, or one within 6 % of it where both are nearly equal.
+bool nh_clu_wins(const pyomgpu_nh* h, size_t ncell) {
+  const double n = (double)ncell;
+  const bool cyclic = h->cyclic_x || h->cyclic_y;
+  double other;
+  if (h->variant == 0 && ncell > (size_t)kNHClusterAuto)
+    other = 8700.0 + (cyclic ? 500.0 : 0.0);
+  else if (ncell <= (size_t)kNHMaxCluster * kNHSmallThreads)
+    other = 6900.0 + 0.073 * n + (cyclic ? 800.0 : 0.0);
+  else
+    other = (ncell <= 2 * (size_t)kNHMaxCluster * kNHSmallThreads ? 7200.0 : 9000.0) + 0.125 * n + (cyclic ? 1100.0 : 0.0);
+  return h->cut.iter_ns < other;
 }
 
 // congrad_non_hydro on device arrays: fdev (forcing) and pdev (p_non_hydro(:,:,:,taup1), in/out), both
@@ -1173,7 +1194,7 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
   // choice is a cluster all the same, as those settings never chose the kernel there
   const bool bricks_asked =
       h->variant == 0 && ncell > (size_t)kNHClusterAuto && (h->grid > 0 || h->ty > 0 || h->ns > 0);
-  if (h->variant != 1 && !bricks_asked && nh_clu_plan(h)) {
+  if (h->variant != 1 && !bricks_asked && nh_clu_plan(h) && nh_clu_wins(h, ncell)) {
     const NHCut& c = h->cut;
     P.cnpx = c.npx;
     P.cnpy = c.npy;
@@ -1188,7 +1209,7 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
     NCK(cudaEventRecord(h->e1, st));
     return nh_finish_cg(h, pdev, info, st);
   }
-  // small grids the cluster kernel's threads or shared memory do not hold (deep or unusually shaped ones)
+  // small grids the cluster kernel's threads or shared memory do not hold, or that it is slower on (deep ones)
   const bool small = h->variant == 2 || (h->variant == 0 && ncell <= (size_t)kNHClusterAuto);
   if (small) {
     // cluster of C = 1, 2, 4, 8 or 16 blocks with about one cell per thread, each chunk within shared memory

@@ -319,6 +319,7 @@ const void* nh_cg_small_kernel_ptr(bool cyclic_x, bool cyclic_y);
 struct NHCut {
   int npx = 0, npy = 0, w = 0, h = 0, p = 0, nt = 0;
   size_t smem = 0;
+  double iter_ns = 0;  // estimated iteration time
 };
 constexpr int kNHCluNP[][2] = {{128, 4}, {128, 8}, {256, 4}, {256, 8}, {256, 12}};  // threads, levels per thread
 // direction with its rim, vertical factors, staged faces, received records (4 words each), reduction slots

@@ -61,7 +61,8 @@ def test_cluster_solve(oracle_lib, nx, ny, nz, cyc_x, cyc_y):
 
 # a level's vertical factors are put into shared memory by one warp and read by others: segments of 4, 8 and 12
 # levels, columns of more levels than a warp has lanes, one block and several
-@pytest.mark.parametrize("nx,ny,nz", [(4, 1, 97), (16, 1, 300), (37, 1, 90), (20, 2, 70), (240, 1, 80), (24, 24, 67)])
+@pytest.mark.parametrize("nx,ny,nz", [(4, 1, 97), (16, 1, 300), (37, 1, 90), (20, 2, 70), (240, 1, 80), (24, 24, 67),
+                                      (96, 4, 100), (60, 60, 12)])
 def test_deep_columns_repeat_to_the_bit(oracle_lib, nx, ny, nz):
     M, forc = tank(nx, ny, nz, False, False)
     O, nh = oracle_lib.Oracle3D(M), NonHydrostatic(M)
@@ -161,4 +162,22 @@ def test_a_nan_ends_the_solve_and_the_halo_keeps_its_offset(oracle_lib, nx, ny, 
         with pytest.raises(_abi.PyOMGPUError) as e:
             nh.congrad_non_hydro(bad, np.zeros(forc.shape, order="F"), eps=1e-9)
         assert e.value.code == _abi.NAN, variant
+    nh.close()
+
+
+# deep narrow tanks, whose faces are large for their cells, are slower in the cluster of whole columns; up to 32768
+# cells they keep the compact cluster, above it the bricks
+@pytest.mark.parametrize("nx,ny,nz,kernel", [
+    (160, 1, 60, "nh_clu_kernel"), (8, 8, 100, "nh_clu_kernel"), (60, 60, 12, "nh_clu_kernel"),
+    (6, 6, 400, "nh_cg_small_kernel"), (8, 8, 400, "nh_cg_small_kernel"), (16, 16, 170, "nh_cg_kernel"),
+    (20, 20, 110, "nh_cg_kernel")])
+def test_deep_tanks_keep_the_kernel_that_is_faster(nx, ny, nz, kernel):
+    from torch.profiler import ProfilerActivity, profile
+    M, forc = tank(nx, ny, nz, False, False)
+    nh = NonHydrostatic(M)
+    with warnings.catch_warnings(), profile(activities=[ProfilerActivity.CUDA]) as p:
+        warnings.simplefilter("ignore")
+        nh.congrad_non_hydro(forc, np.zeros(forc.shape, order="F"), eps=0.0, max_it=3)
+    assert [k for k in ("nh_clu_kernel", "nh_cg_small_kernel", "nh_cg_kernel")
+            if any(k + "<" in e.key for e in p.key_averages())] == [kernel]
     nh.close()
