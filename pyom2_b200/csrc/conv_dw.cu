@@ -95,16 +95,16 @@ __global__ void __launch_bounds__(kDwThreads) conv_dw_kernel(const __grid_consta
   const int px_b = (lane & 7) + (((lane >> 3) & 1) << 3), grp_b = lane >> 4;
   const uint32_t off_a = (uint32_t)((grp_a * kDwBY + dy) * kDwBX + dx + px_a) * 16u;
   const uint32_t off_b = S::GOFF + (uint32_t)(grp_b * kDwRows * kDwCols + px_b) * 16u;
-  float acc[MI][2 * NI][4], accb[2 * NI][4];  // accb: column sums of G, in the warp of tap 0
+  // The matrix unit truncates as it accumulates, so its sums are kept short (the four MMAs of a tile row) and added
+  // up in rounded FP32.  With the accumulators in the MMAs over all tiles the gradients of a 1440x720 image were
+  // 1e-5 too small where all terms have one sign (6e-8 this way; CUDA-core sums scattered by 2.5e-7).
+  float acc[MI][2 * NI][4], accb[2][2] = {};  // accb: warp n has the column sums of G's 16 channels n
 #pragma unroll
-  for (int n = 0; n < 2 * NI; n++) {
-#pragma unroll
-    for (int e = 0; e < 4; e++) accb[n][e] = 0.f;
+  for (int n = 0; n < 2 * NI; n++)
 #pragma unroll
     for (int m = 0; m < MI; m++)
 #pragma unroll
       for (int e = 0; e < 4; e++) acc[m][n][e] = 0.f;
-  }
   const uint32_t kOne = 0x3f803f80u;  // two bf16 ones
   const uint32_t ones[4] = {kOne, kOne, kOne, kOne};
   bool ok = true;
@@ -125,6 +125,13 @@ __global__ void __launch_bounds__(kDwThreads) conv_dw_kernel(const __grid_consta
     const uint32_t s = smem_u32(base + b * S::STAGE);
 #pragma unroll 1
     for (int r = 0; r < kDwRows; r++) {
+      float part[MI][2 * NI][4], partb[2][4] = {};  // sums of one tile row
+#pragma unroll
+      for (int n = 0; n < 2 * NI; n++)
+#pragma unroll
+        for (int m = 0; m < MI; m++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) part[m][n][e] = 0.f;
 #pragma unroll(CIN * COUT <= 512 ? 4 : 1)
       for (int c = 0; c < kDwCols / 16; c++) {
         const uint32_t pa = s + off_a + (uint32_t)(r * kDwBX + 16 * c) * 16u;
@@ -138,18 +145,28 @@ __global__ void __launch_bounds__(kDwThreads) conv_dw_kernel(const __grid_consta
           ldsm4t(pa + (uint32_t)(2 * m * kDwBY * kDwBX) * 16u, fa);
 #pragma unroll
           for (int n = 0; n < NI; n++) {
-            mma16816(acc[m][2 * n], fa, fb[n][0], fb[n][1]);
-            mma16816(acc[m][2 * n + 1], fa, fb[n][2], fb[n][3]);
+            mma16816(part[m][2 * n], fa, fb[n][0], fb[n][1]);
+            mma16816(part[m][2 * n + 1], fa, fb[n][2], fb[n][3]);
           }
         }
-        if (warp == 0) {
 #pragma unroll
-          for (int n = 0; n < NI; n++) {
-            mma16816(accb[2 * n], ones, fb[n][0], fb[n][1]);
-            mma16816(accb[2 * n + 1], ones, fb[n][2], fb[n][3]);
+        for (int n = 0; n < NI; n++)
+          if (warp == n) {
+            mma16816(partb[0], ones, fb[n][0], fb[n][1]);
+            mma16816(partb[1], ones, fb[n][2], fb[n][3]);
           }
-        }
       }
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        accb[q][0] += partb[q][0];
+        accb[q][1] += partb[q][1];
+      }
+#pragma unroll
+      for (int n = 0; n < 2 * NI; n++)
+#pragma unroll
+        for (int m = 0; m < MI; m++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) acc[m][n][e] += part[m][n][e];
     }
     __syncthreads();
   }
@@ -171,11 +188,11 @@ __global__ void __launch_bounds__(kDwThreads) conv_dw_kernel(const __grid_consta
         const int ci = 16 * m + (lane >> 2) + 8 * (e >> 1), co = 8 * n + 2 * (lane & 3) + (e & 1);
         atomicAdd(a.dW + ((size_t)(co0 + co) * CIN + ci) * 9 + warp, acc[m][n][e]);
       }
-  if (warp == 0 && lane < 4)  // every row of accb holds the sums
+  if (warp < NI && lane < 4)  // every row of accb holds the sums
 #pragma unroll
-    for (int n = 0; n < 2 * NI; n++) {
-      atomicAdd(a.db + co0 + 8 * n + 2 * lane, accb[n][0]);
-      atomicAdd(a.db + co0 + 8 * n + 2 * lane + 1, accb[n][1]);
+    for (int q = 0; q < 2; q++) {
+      atomicAdd(a.db + co0 + 16 * warp + 8 * q + 2 * lane, accb[q][0]);
+      atomicAdd(a.db + co0 + 16 * warp + 8 * q + 2 * lane + 1, accb[q][1]);
     }
 }
 

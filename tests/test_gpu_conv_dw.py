@@ -102,3 +102,34 @@ def test_output_layer_gradient_to_fp32(nx, ny):
     assert np.all(got[1:] == 0.0)
     assert abs(g[o + off[11]] - gb.sum()) <= 1e-5 * np.abs(gb).sum()
     pc.close()
+
+
+def test_sums_do_not_drift():
+    """The gradient of the output layer against the exact sums of the same bf16 operands, all positive, so that a
+    rounding of one sign in the accumulation adds up.  Sums of four products of 16 pixels each may be truncated
+    (on average half a unit of 2**-23 of the running sum, at most a whole one): the mean error is at most
+    (1/4 + 2/4 + 3/4 + 1) 2**-24 2 = 3e-7 of the sum, and half of that expected; rounded sums on top of them (four
+    a tile of 4 x 64 pixels and one a block) scatter by less than sqrt(400) 2**-24 and have no mean."""
+    nx, ny = 1440, 720
+    sl, _ = layer_slices()
+    p = np.zeros(learned.num_params(), dtype=np.float32)
+    for k in (0, 1):  # the first level's activations are the input, the coarser levels add nothing
+        w = np.zeros(sl[k][1], dtype=np.float32)
+        w[np.arange(16), np.arange(16), 1, 1] = 1.0
+        p[sl[k][0]] = w.ravel()
+    pc = trainer(nx, ny, p)
+    rng = np.random.default_rng(2)
+    x = U.bf16_round(rng.uniform(0.5, 1.5, (16, ny, nx)))
+    gz = np.abs(rng.standard_normal((ny, nx))).astype(np.float32)
+    pc.forward_backward(U.bf16_bits(U.to_planar(x)), gz)
+    s, shape = sl[11]
+    got = pc.get_grads()[s].reshape(shape)[0].astype(np.float64)
+    pc.close()
+    xp, g = np.pad(x, ((0, 0), (1, 1), (1, 1))), U.bf16_round(gz.astype(np.float64))
+    want = np.empty((16, 3, 3))
+    for dy in range(3):
+        for dx in range(3):
+            want[:, dy, dx] = (xp[:, dy:dy + ny, dx:dx + nx] * g).sum(axis=(1, 2))
+    err = got / want - 1.0
+    assert abs(err.mean()) <= 2.5 * 2.0 ** -23
+    assert err.std() <= 20 * 2.0 ** -24
