@@ -478,7 +478,8 @@ int32_t pyomgpu_nh_inject_barrier_stall(pyomgpu_nh* nh, int32_t enable);
  * level. */
 int32_t pyomgpu_nh_set_grid(pyomgpu_nh* nh, int32_t blocks);
 /* Brick shape of the CG sweeps: 32 x ty x kc cells staged with their halo in
- * shared memory (0, 0 = automatic: ty = min(8, ny), kc from a 26 KB box). */
+ * shared memory (0, 0 = automatic: ty the largest power of two up to
+ * min(8, ny), kc the height whose busiest block has the least to do). */
 int32_t pyomgpu_nh_set_brick(pyomgpu_nh* nh, int32_t ty, int32_t kc);
 /* TMA pipeline depth of the CG sweeps: 2..4 stages (0 = automatic, 2). */
 int32_t pyomgpu_nh_set_stages(pyomgpu_nh* nh, int32_t stages);

@@ -14,9 +14,9 @@
 //     cluster reads its warps' partials instead);
 //   * the boundary values (Z res, direction) go from the owning thread's
 //     registers into the neighbour's inbox, in the sweep that makes them;
-//   * all sixteen warps own points (column segments of P rows, as in
-//     cg_res.cu): residual, direction and Z*res (or A s) in registers, the
-//     solution and Z too up to P = 4, else in shared memory.
+//   * all warps (four or eight a block) own points, column segments of P rows
+//     as in cg_res.cu: residual, direction, Z*res (or A s), solution and Z in
+//     registers, the face couplings too up to P = 4, else in shared memory.
 // An inbox word is rewritten only after every reader has passed it: a slot of
 // epoch e at e+2, when every block has published e+1; a halo record one
 // iteration later, when its reader has published the sweep A in between.

@@ -41,8 +41,10 @@ __device__ __forceinline__ T* res_resv(const CGResParams& P) {
 }
 
 // ------------------------------------------------------------ control flow
-// Scalars of the solve in shared memory, advanced by thread 0 only (the
-// reference's congrad_streamfunction variables).
+// Scalars of the solve (the reference's congrad_streamfunction variables).  In
+// the resident kernels one copy in shared memory, advanced by one thread; in
+// the cluster kernel every thread keeps a copy and advances it, so there the
+// reduced values must have the same bits in every thread of the cluster.
 struct ResCtl {
   double beta, bb, rtol2bb, betam1, betamin, step1, est, bq, alpha;
   int n, status, act, stop_after;

@@ -953,7 +953,7 @@ __device__ __forceinline__ void res_solve(const CGResParams& Pm, const int bid, 
       {
         const int sp = opaque(pw + 2);
         const T bq = (T)C.bq;
-T* o = ss + (ly0 + 1) * sp + lx + 1;
+        T* o = ss + (ly0 + 1) * sp + lx + 1;
 #pragma unroll
         for (int u = 0; u < P; u++) {
           s[u] = q[u] + bq * s[u];
@@ -973,7 +973,9 @@ T* o = ss + (ly0 + 1) * sp + lx + 1;
         double v[2] = {0.0, 0.0};  // (s, As), max|s|
         if (nrow > 0) {
           // No branch per point: with one, a point's loads and its chain of a dozen FP64 operations ran before
-          // the next point's began.  Rows past the segment repeat its last one and are dropped from the sums.
+          // the next point's began.  Rows past the segment (u >= nrow) use its last row's couplings with an s[u] of
+          // their own, so A s and the residual hold values of no meaning there, with SP the direction too (else
+          // Z = 0 keeps it 0): every sum, staged value and store has to select on u < nrow.
           const T *o = ss + (ly0 + 1) * sp + lx + 1, *fx = sfx + ly0 * (pw + 1) + lx, *fy = sfy + (ly0 + 1) * pw + lx;
           const T *bx = sbx + ly0, *by = sbx + ph + ly0;
           const T below = o[-sp], above = o[nrow * sp];

@@ -8,9 +8,9 @@
 // matrix (8 rows x 16 bytes), so a TMA-loaded input box is a valid K-major
 // MMA operand for every one of the 9 taps by an address offset alone.
 //
-// Weights are packed once per update as [tap][Cin/8][Cout][8] bf16 (the
-// shared-memory image of the B operand); PyTorch's [Cout][Cin][3][3] order
-// is the interchange format.
+// Weights are packed once per update as [dx][Cin/8][2-dy][Cout][8] bf16 (the
+// shared-memory image of the B operand: the three dy of a dx side by side in
+// N); PyTorch's [Cout][Cin][3][3] order is the interchange format.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -1087,8 +1087,9 @@ void nh_clu_config(const NHCut& c, cudaLaunchConfig_t& cfg, cudaLaunchAttribute&
 // 256/12 on 16 5.53; 64 x 1 x 24 one block 256/8 1.69, two of 256/4 2.41;
 // 40 x 24 x 10 256/4 on 6 x 2, 4 x 3 3.73, 4.03; 40 x 36 x 9 256/8 on 2 x 6,
 // 4 x 3, 14 x 1 4.67, 5.08, 5.72; 48 x 40 x 24 256/12 on 8 x 2, 16 x 1 9.06,
-// 11.42.  (Opposite faces have since come to share a pass; the chosen cuts run
-// 0.2 to 0.5 faster than these.)
+// 11.42.  Opposite faces have since come to share a pass, which took 0.2 to 0.5
+// from those cuts; deep narrow ones (14 x 14 x 160: 13.1 estimated, 14.7) are
+// up to 12 % above the estimate.
 double nh_clu_iter_ns(const pyomgpu_nh* h, int npx, int npy, int w, int hh, int p, int nt) {
   const int nz = h->G.nz, nb = npx * npy;
   if (nb == 1) return 1000.0 + 85.0 * p;
@@ -1105,7 +1106,7 @@ double nh_clu_iter_ns(const pyomgpu_nh* h, int npx, int npy, int w, int hh, int 
 // cuts in x and y into at most kCluMaxBlocks pieces of whole columns that fit
 // its threads and shared memory, the one with the smallest estimated iteration
 // time.  False where none fits (about 49 000 cells at most) or the device
-// cannot place the cluster.
+// cannot place the cluster.  Whether it is run is nh_clu_wins's to say.
 bool nh_clu_plan(pyomgpu_nh* h) {
   NHCut& best = h->cut;
   if (h->cut_planned) return best.npx > 0;

@@ -93,14 +93,6 @@ __device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* m
 __device__ __forceinline__ void st_hint(double* p, double v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol) : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-      : "memory");
-}
 
 // Host: tensor map of a padded FP64 field ((ny+4) rows of `pitch` elements)
 // with a box_x x box_y box.  Returns 0 or a CUDA driver error code.

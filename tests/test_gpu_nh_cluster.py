@@ -1,6 +1,6 @@
 """Small non-hydrostatic grids in one thread-block cluster (nh_clu.cu): the automatic kernel choice
-against the oracle, from one block of a few cells to the largest cluster and beyond it; and the
-warp-uniform fast paths of the brick kernel (all faces, none, mixed) on the same problems."""
+and the brick kernel against the oracle, from one block of a few cells to the largest cluster and
+beyond it; the compact cluster kernel where that is the choice; and which kernel is."""
 import warnings
 
 import numpy as np
