@@ -112,8 +112,10 @@ struct NHPipe {
 // of a 240 x 240 x 80 tank (111 MB) just fit in L2; walked in one direction
 // every time they evicted themselves (DRAM bytes equal to the algorithmic 66
 // per cell, 77.7 us per iteration), walked back and forth each sweep starts on
-// what the last one left.  p, which only sweep B touches, passes through with
-// an evict-first policy.
+// what the last one left.  (With an evict-first policy for p, which only sweep B
+// touches, it was slower: 76.2 us against 75.8 here, 149 against 144 at
+// 300 x 300 x 100, 589 against 546 at 480 x 480 x 160, 14.0 against 13.8 at
+// 75 x 69 x 61.)
 //   sweep A (kB false): stage = s_{n-1} box (buffer cur), res box, flags;
 //   sweep B (kB true):  stage = s_n box (buffer cur ^ 1), the brick's res
 //     and p, flags.
@@ -140,7 +142,6 @@ __device__ __forceinline__ bool nh_sweep(const NHParams& P, int cur, double bq, 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int jj = warp % TY, kk0 = (warp / TY) * KW;
   const int nmine = (int)blockIdx.x < nbr ? (nbr - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const uint64_t pol = kB ? l2_evict_first() : 0;
   // thread 0: put brick number m of this block into stage st once the stage is free
   auto produce = [&](int m, int st) -> bool {
     if (pp.used & (1u << st)) {
@@ -164,7 +165,7 @@ __device__ __forceinline__ bool nh_sweep(const NHParams& P, int cur, double bq, 
     } else {  // box 0 = s_n, then the brick's res and p
       tma_load_3d(B, &P.map_s[cur ^ 1], x, y, z, &pp.full[st]);
       tma_load_3d(B + rs, &P.map_res_brick, xb, yb, zb, &pp.full[st]);
-      tma_load_3d_hint(B + rs + pb, &P.map_p, xb, yb, zb, &pp.full[st], pol);
+      tma_load_3d(B + rs + pb, &P.map_p, xb, yb, zb, &pp.full[st]);
     }
     // flags: column i0-1 (a multiple of 32 bytes), row j0-1, level k0-1
     tma_load_3d(B + fo, &P.map_f, 32 * bx, TY * by, KC * bz, &pp.full[st]);
@@ -334,7 +335,6 @@ __global__ void __launch_bounds__(kNHThreads, 2) nh_cg_kernel(const __grid_const
     if (how != NHCtl::kGo) break;
     // -------------------------------------------------------------- sweep B
     double acc_r = 0.0;
-    const uint64_t pol = l2_evict_first();
     const bool ok = nh_sweep<true>(
         P, cur, ctl.bq, smem, pp,
         [&](int i, int j, int, uint32_t f, size_t q, double a, double sc, double rc, double pc) {
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kNHThreads, 2) nh_cg_kernel(const __grid_const
           const double d = __dmul_rn(alpha, sc);                // p_non_hydro + alpha*p (:187)
           ptrdiff_t ox, oy;
           nh_copy_offsets<CX, CY>(G.g, i, j, ox, oy);
-          st_hint(pnh + q, __dadd_rn(pc, d), pol);
+          pnh[q] = __dadd_rn(pc, d);
           nh_add_halo<CX, CY>(pnh, q, ox, oy, d);
           nh_put<CX, CY>(res, q, ox, oy, r);
           if (f & kNHMaskT) acc_r += r * r;

@@ -75,25 +75,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-// L2 policy for data read or written once before everything else passes
-// through: it is the first to leave, so it displaces nothing that comes back.
-__device__ __forceinline__ uint64_t l2_evict_first() {
-  uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-  return pol;
-}
-__device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                                 uint64_t* bar, uint64_t pol) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], "
-      "[%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)), "l"(pol)
-      : "memory");
-}
-__device__ __forceinline__ void st_hint(double* p, double v, uint64_t pol) {
-  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol) : "memory");
-}
-
 // Host: tensor map of a padded FP64 field ((ny+4) rows of `pitch` elements)
 // with a box_x x box_y box.  Returns 0 or a CUDA driver error code.
 int encode_tile_map(CUtensorMap* map, const double* base, const Geo& g, int box_x = kBoxX, int box_y = kBoxY);
