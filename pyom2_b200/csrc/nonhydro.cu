@@ -1251,9 +1251,12 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
   // largest level count per warp kw whose pipeline stages leave room for two blocks per SM.  Of these kw the one
   // whose busiest block has the least to do, a brick costing about its levels and two more: a short last round
   // of bricks, or idle SMs, cost more than flatter bricks' wider halos.  us per iteration, kc = 7 and the choice:
-  // 60 x 60 x 20 10.86, 8.78 (3); 100 x 100 x 30 13.66, 13.07 (6); 120 x 120 x 40 18.31, 16.65 (5);
-  // 180 x 180 x 60 36.2, 35.5 (6); 240 x 240 x 80 keeps 7 (74.2; 77.6 with 5).  Fewer than 3 levels a warp lose
-  // to the march's start (60 x 60 x 20: 9.38 with 2).
+  // 60 x 60 x 20 10.58, 8.61 (3); 100 x 100 x 30 13.52, 13.20 (6); 120 x 120 x 40 18.54, 16.53 (5);
+  // 180 x 180 x 60 37.4, 36.5 (6); 240 x 240 x 80 keeps 7 (75.9; 78.2 with 5).  Fewer than 3 levels a warp lose
+  // to the march's start (60 x 60 x 20: 9.40 with 2).  The estimate is no better than 5 %, and the tallest bricks
+  // read the fewest halos, so they stay unless another height is that much below (234 x 179 x 23, cyclic: 27.6 us
+  // with 4, estimated 24 against 27, 26.5 with 6, 25.9 with 7; 300 x 300 x 100: 6 and 7 estimated 176 and 180,
+  // 7 2 % faster).
   int ty = h->ty, kc = h->kc, ns = h->ns > 0 ? h->ns : 2;
   if (ty == 0) {
     ty = h->G.g.ny >= 8 ? 8 : h->G.g.ny >= 4 ? 4 : h->G.g.ny >= 2 ? 2 : 1;
@@ -1263,15 +1266,16 @@ int nh_run_cg(pyomgpu_nh* h, const double* fdev, double* pdev, double eps, int m
     int kw0 = std::min(3, kw_need);
     while (kw0 > 1 && !fits(kw0)) kw0--;
     const long long cols = (long long)((h->G.g.nx + 31) / 32) * ((h->G.g.ny + ty - 1) / ty);
-    long long least = 0;
-    for (int kw = kw0; kw <= kw_need && (kw == kw0 || fits(kw)); kw++) {
+    int top = kw0;
+    while (top < kw_need && fits(top + 1)) top++;
+    auto cost = [&](int kw) {
       const long long bricks = cols * ((h->G.nz + seg * kw - 1) / (seg * kw));
-      const long long cost = (bricks + nblk - 1) / nblk * (kw + 2);
-      if (kw == kw0 || cost < least) {
-        kc = seg * kw;
-        least = cost;
-      }
-    }
+      return (bricks + nblk - 1) / nblk * (kw + 2);
+    };
+    int best = top;
+    for (int kw = top - 1; kw >= kw0; kw--)
+      if (cost(kw) < cost(best) && 20 * cost(kw) < 19 * cost(top)) best = kw;
+    kc = seg * best;
   }
   while (ns > 2 && nh_smem_bytes(ty, kc, ns) > kNHSmemMax) ns--;
   const size_t smem = nh_smem_bytes(ty, kc, ns);
