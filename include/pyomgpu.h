@@ -479,7 +479,8 @@ int32_t pyomgpu_nh_inject_barrier_stall(pyomgpu_nh* nh, int32_t enable);
 int32_t pyomgpu_nh_set_grid(pyomgpu_nh* nh, int32_t blocks);
 /* Brick shape of the CG sweeps: 32 x ty x kc cells staged with their halo in
  * shared memory (0, 0 = automatic: ty the largest power of two up to
- * min(8, ny), kc the height whose busiest block has the least to do). */
+ * min(8, ny), kc the tallest that two blocks per SM have room for, or a lower
+ * one with which the busiest block has clearly less to do). */
 int32_t pyomgpu_nh_set_brick(pyomgpu_nh* nh, int32_t ty, int32_t kc);
 /* TMA pipeline depth of the CG sweeps: 2..4 stages (0 = automatic, 2). */
 int32_t pyomgpu_nh_set_stages(pyomgpu_nh* nh, int32_t stages);
